@@ -2,7 +2,7 @@
 (pass1, accumulate_profiles, pass2) with the reference's signatures and dict results
 (`xpg/integrate_kernels.py:216-485`), for callers that drive the kernels themselves.
 
-Arguments are torch CUDA tensors (numpy arrays are moved to the device): `sb` (N, Dz, Dy, Dx) float32 shoeboxes
+Arguments are torch CUDA tensors, read where they are (anything else is moved to the device): `sb` (N, Dz, Dy, Dx) float32 shoeboxes
 (values, -1 masked, -2 overloaded, -3 unrecorded), the `rc` dict (S, phi, ix0, iy0, iz0, fb, region, has_p, pS, pphi
 and optionally pxs), the `nb` dict (x, y, z, sx, sz: (N, K)), and `det` from `detector_consts(geometry,
 bkg_template)` (XPG's `_detector_consts`). `axis`, `s0`, `frames_phi0`, `osc`, `sd`, `sm`, `gain` and `rcw` as in the
@@ -30,13 +30,25 @@ def _np(v):
     return np.asarray(v)
 
 
+def _in(v):
+    """A per-row or per-pixel argument for `device._dev`: a CUDA tensor as it is (it is converted on the device, or
+    read in place), anything else as a numpy array. Through the host instead, the pixel tables' copies alone took
+    most of a call (4096 boxes of 31 x 31 x 33: 26.3 ms for the three passes, 3.8 ms of it kernels)."""
+    return v.detach() if torch.is_tensor(v) and v.is_cuda else _np(v)
+
+
+def _on_device(v):
+    """The argument's values as a device tensor, in its own shape."""
+    t = _in(v)
+    return t.to("cuda") if torch.is_tensor(t) else torch.as_tensor(t).to("cuda")
+
+
 def _rows(sb, rc, nb, Dz, Dx):
     n = int(sb.shape[0])
-    pxs = _np(rc["pxs"]).astype(np.int32) if "pxs" in rc else np.ones(n, np.int32)
-    return D.RowSet(S=_np(rc["S"]), phi=_np(rc["phi"]), ix0=_np(rc["ix0"]), iy0=_np(rc["iy0"]), iz0=_np(rc["iz0"]),
-                    fb=_np(rc["fb"]), region=_np(rc["region"]), has_p=_np(rc["has_p"]), pS=_np(rc["pS"]),
-                    pphi=_np(rc["pphi"]), pxs=pxs, Dz=np.full(n, Dz), bx=np.full(n, Dx),
-                    nb={k: _np(nb[k]) for k in ("x", "y", "z", "sx", "sz")}, sb_bias=0.0)
+    one = ("S", "phi", "ix0", "iy0", "iz0", "fb", "region", "has_p", "pS", "pphi")
+    pxs = _in(rc["pxs"]) if "pxs" in rc else np.ones(n, np.int32)
+    return D.RowSet(**{k: _in(rc[k]) for k in one}, pxs=pxs, Dz=np.full(n, Dz), bx=np.full(n, Dx),
+                    nb={k: _in(nb[k]) for k in ("x", "y", "z", "sx", "sz")}, sb_bias=0.0)
 
 
 def _block(axis, s0, frames_phi0, osc, sd, sm, gain, rcw):
@@ -49,6 +61,11 @@ def _block(axis, s0, frames_phi0, osc, sd, sm, gain, rcw):
     for c in range(3):
         b.axis[c], b.s0[c] = float(a[c]), float(s[c])
     return b, rc
+
+
+def _groups(rows):
+    """One launch over the rows in order: they have one shape."""
+    return [(int(rows.bx[0]), int(rows.Dz[0]), None)] if rows.n else []
 
 
 def _sb(sb):
@@ -69,7 +86,7 @@ def make_kernels(Dz, Dy, Dx, n_regions, G=PROFILE_GRID):
         blk, keep = _block(axis, s0, frames_phi0, osc, sd, sm, gain, rcw)
         arena = _sb(sb)
         out = D.Pass1Buffers(rows)
-        D.pass1(det, rows, blk, arena, out)
+        D.pass1(det, rows, blk, arena, out, groups=_groups(rows))
         D.status()
         t = out.t
         n = rows.n
@@ -91,22 +108,22 @@ def make_kernels(Dz, Dy, Dx, n_regions, G=PROFILE_GRID):
         n = int(img2.shape[0])
         nbz = {k: np.zeros((n, 1), np.float32) for k in ("x", "y", "z", "sx", "sz")}
         rc = dict(S=np.zeros((n, 3), np.float32), phi=np.zeros(n, np.float32), ix0=np.zeros(n, np.int32),
-                  iy0=np.zeros(n, np.int32), iz0=np.zeros(n, np.int32), fb=np.ones(n, np.float32), region=_np(region),
+                  iy0=np.zeros(n, np.int32), iz0=np.zeros(n, np.int32), fb=np.ones(n, np.float32), region=_in(region),
                   has_p=np.zeros(n, np.float32), pS=np.zeros((n, 3), np.float32), pphi=np.zeros(n, np.float32))
         rows = _rows(np.zeros((n, 1, Dy, Dx), np.float32), rc, nbz, 1, Dx)
         buf = D.Pass1Buffers(rows)
-        f = lambda v: torch.as_tensor(_np(v)).to("cuda")
-        buf.t["img2"].copy_(f(img2).reshape(-1).float())
-        buf.t["all_valid2"].copy_(f(ok2).reshape(-1).to(torch.uint8))
-        buf.t["J"].copy_(f(J).reshape(-1).float())
-        buf.t["u1"].copy_(f(u1).reshape(-1).float())
-        buf.t["u2"].copy_(f(u2).reshape(-1).float())
-        buf.t["isum"].copy_(f(isum).float())
-        buf.t["seff"].copy_(f(seff).float())
+        for k, v in (("img2", img2), ("J", J), ("u1", u1), ("u2", u2)):
+            buf.t[k].copy_(_on_device(v).reshape(-1).float())
+        buf.t["all_valid2"].copy_(_on_device(ok2).reshape(-1).to(torch.uint8))
+        buf.t["isum"].copy_(_on_device(isum).float())
+        buf.t["seff"].copy_(_on_device(seff).float())
         num = torch.zeros((n_regions, G, G), dtype=torch.float64, device="cuda")
         den = torch.zeros_like(num)
-        selt = f(sel).to(torch.uint8).contiguous()
+        selt = _on_device(sel).to(torch.uint8).contiguous()
         D.accumulate(rows, buf, n_regions, num, den, sel=selt, strong_test=False)
+        for v in (img2, ok2, J, u1, u2, region, isum, sel, seff):      # read behind the call's return
+            if torch.is_tensor(v) and v.is_cuda:
+                v.record_stream(torch.cuda.current_stream(v.device))
         return num, den
 
     def pass2(sb, rc, det, axis, s0, frames_phi0, osc, sd, sm, gain, prof, bg, nbm_x, nb, rcw, pix=None):
@@ -118,15 +135,12 @@ def make_kernels(Dz, Dy, Dx, n_regions, G=PROFILE_GRID):
             r1 = pass1(sb, rc, det, axis, s0, frames_phi0, osc, sd, sm, gain, prof, nb, rcw)
             pix = {k: r1[k] for k in ("zeta", "J", "u1", "u2", "seff")}
         buf = D.Pass1Buffers(rows)
-        f = lambda v: torch.as_tensor(_np(v)).to("cuda").reshape(-1).float()
-        for k in ("zeta", "seff", "J", "u1", "u2"):
-            buf.t[k].copy_(f(pix[k]))
-        buf.t["bg"].copy_(f(bg))
-        buf.t["nbg"].copy_(f(nbm_x))
+        for k, v in (*((k, pix[k]) for k in ("zeta", "seff", "J", "u1", "u2")), ("bg", bg), ("nbg", nbm_x)):
+            buf.t[k].copy_(_on_device(v).reshape(-1).float())
         blk, keep = _block(axis, s0, frames_phi0, osc, sd, sm, gain, rcw)
         out = D.Pass2Buffers(rows)
-        proft = torch.as_tensor(_np(prof).astype(np.float32)).cuda().contiguous()
-        D.pass2(det, rows, blk, arena, proft, buf, out)
+        proft = _on_device(prof).float().contiguous()
+        D.pass2(det, rows, blk, arena, proft, buf, out, groups=_groups(rows))
         D.status()
         return dict(out.t)
 
