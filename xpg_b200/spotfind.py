@@ -36,7 +36,7 @@ def make_finder(nbx=3, nby=3, signal_pixel=3.0, background_pixel=2.0, min_local=
         ws = torch.empty(max(nws, 1), dtype=torch.uint8, device=x.device)
         N.check(lib.xi_spot_strong(N.ptr(x), B, ny, nx, float(gain), C.byref(p), N.ptr(strong), N.ptr(mean),
                                    N.ptr(ws), nws, N.stream_handle()), "xi_spot_strong")
-        return strong.bool().reshape(shape), mean.reshape(shape)
+        return strong.view(torch.bool).reshape(shape), mean.reshape(shape)
 
     return find
 
