@@ -115,6 +115,7 @@ __device__ inline void pixel_S(const XiDetector& d, float x, float y, float S[3]
             U2[c] = d.U2[3 * k + c];
             UN[c] = d.UN[3 * k + c];
         }
+#pragma unroll 1
         for (int it = 0; it < 2; ++it) {
             float n = norm3(X[0], X[1], X[2]);
             float e[3] = {X[0] / n, X[1] / n, X[2] / n};
@@ -166,23 +167,6 @@ __device__ __forceinline__ float box_coord(int i0, int i, int pxs) {
         return (((float)i0 + (float)i) * s + (s - 1.0f) * 0.5f) + 1.0f;
     }
     return ((float)i0 + (float)i) + 1.0f;
-}
-
-// rocking-curve mixture fraction of one frame bin (xpg/integrate_kernels.py:130-141, :255-262); the 21 terms are
-// summed in float64 in component order and rounded once
-__device__ inline float rocking_fraction(float lo, float hi, float phi, float zeta, float sm, const float* rcw) {
-    float s = sm / fmaxf(fabsf(zeta), 1e-3f);
-    float sw = (s * 0.25f) * kSqrt2;
-    double acc = 0.0;
-    for (int k = 0; k < XI_RC_K; ++k) {
-        float c = (k == XI_RC_K - 1) ? 3.5f : (float)((double)k * 0.35 + (-3.5));
-        float cs = c * s;
-        float a = ((hi - phi) - cs) / sw;
-        float b = ((lo - phi) - cs) / sw;
-        float term = (rcw[k] * 0.5f) * (erf32(a) - erf32(b));
-        acc += (double)term;
-    }
-    return (float)acc;
 }
 
 // frame bin limits (xpg/integrate_kernels.py:256-260)
@@ -285,12 +269,6 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
 // reductions
 // ------------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
-}
-
-__device__ __forceinline__ float warp_sumf(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     return v;
