@@ -409,7 +409,13 @@ constexpr int kClipCand = 1024;     // background voxels above the lowest clip t
 constexpr int kFgList = 2048;       // foreground pixels listed per CTA (pass C iterates them densely), at most
 constexpr int kClipWarp = 256;      // candidates that one warp iterates alone
 constexpr int kZBatch = 8;          // voxels of a pixel column loaded together (memory-level parallelism)
-constexpr int kGatherBatch = 8;     // frames of a box pixel read together by the gather
+// The gather's threads per row and the frames of a box pixel that a thread reads together. Bound by memory latency
+// (15 of 20 stall cycles) and by how many frames' pages are open at once: more frames in flight a thread make it slower
+// (16 frames: 16.7 ms for the 16M-pixel sweep's 107,446 rows), more pixels of the same frames faster. 128 threads and
+// 8 frames: 5.94 ms there and 5.10 ms for the 4M-pixel sweep's 90,287; 256 and 4: 5.06 and 4.44 ms; 512 and 4: 4.80 and
+// 4.96 ms.
+constexpr int kGatherThreads = 256;
+constexpr int kGatherBatch = 4;
 
 // Dynamic shared memory of pass 1 for boxes up to max_bx pixels a side and max_dz bins with K neighbour columns: the
 // neighbours' frame masks (8P) | geometry scratch eps1, then the background template (4P) | eps2, then the img2 counts
@@ -2163,7 +2169,7 @@ int xi_gather(const XiFrames* F, const XiGatherRows* G, float* arena, int32_t* c
     if (F->n_frames < 0 || F->ny <= 0 || F->nx <= 0 || G->n < 0) return fail(XI_E_ARG, "xi_gather: bad sizes");
     const int nblk = G->order ? G->n_order : G->n;
     if (nblk == 0 || F->n_frames == 0) return XI_OK;
-    k_gather<<<nblk, 128, 0, (cudaStream_t)stream>>>(*F, *G, arena, cnt, G->order);
+    k_gather<<<nblk, kGatherThreads, 0, (cudaStream_t)stream>>>(*F, *G, arena, cnt, G->order);
     return cuda_check("xi_gather");
 }
 
@@ -2171,7 +2177,7 @@ int xi_gather_step(const XiGatherStep* step, const XiGatherRows* G, float* arena
                    void* stream) {
     if (!step || !G || !arena) return fail(XI_E_ARG, "xi_gather_step: null argument");
     if (grid <= 0 || G->n < 0) return fail(XI_E_ARG, "xi_gather_step: bad sizes");
-    k_gather_step<<<grid, 128, 0, (cudaStream_t)stream>>>(step, *G, arena, cnt);
+    k_gather_step<<<grid, kGatherThreads, 0, (cudaStream_t)stream>>>(step, *G, arena, cnt);
     return cuda_check("xi_gather_step");
 }
 
