@@ -1,5 +1,5 @@
-"""Pass 1 and pass 2 at the shapes where their loops end unevenly (frame batches of eight, runs of nine, words of 32
-frames, boxes of fewer or slightly more pixels than a CTA has threads), with the box staged or not, both CTA widths and
+"""Pass 1 and pass 2 at the shapes where their loops end unevenly (frame batches of eight, nine and seventeen, runs of
+nine, boxes of fewer or slightly more pixels than a CTA has threads), with the box staged or not, both CTA widths and
 a fit list that holds all, some or none of the fitted voxels, against the oracle: masks, counts and per-pixel terms bit
 for bit, sums within 1e-5 (pass 1) and 2e-6 (pass 2) of their scale, as for the stored chunks."""
 from __future__ import annotations
@@ -55,7 +55,7 @@ def tuned():
     yield tune
     for key, value in ((N.XI_TUNE_WIDE_THREADS, 256), (N.XI_TUNE_PASS1_STAGE_BYTES, 48 * 1024),
                        (N.XI_TUNE_PASS2_STAGE_BYTES, 48 * 1024), (N.XI_TUNE_PASS2_LIST_CAP, 2048),
-                       (N.XI_TUNE_PASS2_LIST_CAP_LARGE, 8192)):
+                       (N.XI_TUNE_PASS2_LIST_CAP_LARGE, 2048)):
         N.check(lib.xi_tune(key, value), "xi_tune")
     N._apply_tuned(lib)
 

@@ -38,8 +38,8 @@ constexpr float kSbOff = 3.0f;     // shoeboxes are stored as value + 3 (0 = unr
 // neighbour data of a CTA: per active neighbour, squared normalised distances per column / row / frame
 struct NbShared {
     int nact;
-    int act[XI_MAX_K];
     int zmin[XI_MAX_K];             // frame of the smallest dz^2 of each active neighbour
+    float x[XI_MAX_K], y[XI_MAX_K], z[XI_MAX_K], sx[XI_MAX_K], sz[XI_MAX_K];
 };
 
 // The per-axis terms of the active neighbours, in dynamic shared memory sized for the launch's neighbour columns
@@ -94,25 +94,31 @@ __device__ __forceinline__ void neighbour_test(const NbColumn& c, int K, bool sk
         on = (mx * mx + my * my) + mz * mz < 1.0f;
     }
     const unsigned ball = __ballot_sync(0xffffffffu, on);
-    if (on) nb.act[__popc(ball & ((1u << k) - 1u))] = k;
+    if (on) {
+        const int a = __popc(ball & ((1u << k) - 1u));
+        nb.x[a] = c.x;
+        nb.y[a] = c.y;
+        nb.z[a] = c.z;
+        nb.sx[a] = c.sx;
+        nb.sz[a] = c.sz;
+    }
     if (k == 0) nb.nact = __popc(ball);
 }
 
-// The active neighbours' per-axis terms, by the whole CTA (no barrier).
-__device__ __forceinline__ void neighbour_axes(const XiRows& R, int row, int Dz, int bx, const float* xs,
-                                               const float* ys, int iz0, float fb, const NbShared& nb,
-                                               const NbTab& tb) {
-    for (int a = 0; a < nb.nact; ++a) {
-        NbColumn c;
-        c.load(R, row, nb.act[a]);
-        for (int i = threadIdx.x; i < bx; i += blockDim.x) {
-            const float dx = (xs[i] - c.x) / c.sx;
-            const float dy = (ys[i] - c.y) / c.sx;
-            tb.x2(a, i) = dx * dx;
-            tb.y2(a, i) = dy * dy;
-        }
-        for (int z = threadIdx.x; z < Dz; z += blockDim.x) {
-            const float dz = (frame_centre(iz0, fb, z) - c.z) / c.sz;
+// The active neighbours' per-axis terms, spread over the CTA (no barrier).
+__device__ __forceinline__ void neighbour_axes(int Dz, int bx, const float* xs, const float* ys, int iz0, float fb,
+                                               const NbShared& nb, const NbTab& tb) {
+    const int each = 2 * bx + Dz;
+    for (int q = threadIdx.x; q < nb.nact * each; q += blockDim.x) {
+        const int a = q / each, e = q - a * each;
+        if (e < 2 * bx) {
+            const bool col = e < bx;
+            const int i = col ? e : e - bx;
+            const float d = ((col ? xs[i] : ys[i]) - (col ? nb.x[a] : nb.y[a])) / nb.sx[a];
+            (col ? tb.x2(a, i) : tb.y2(a, i)) = d * d;
+        } else {
+            const int z = e - 2 * bx;
+            const float dz = (frame_centre(iz0, fb, z) - nb.z[a]) / nb.sz[a];
             tb.z2(a)[z] = dz * dz;
         }
     }
@@ -178,7 +184,10 @@ __device__ __forceinline__ Mask65 neighbour_frames(const NbShared& nb, const NbT
     return m;
 }
 
-__device__ __forceinline__ unsigned pick3(const unsigned (&m)[3], int w) { return w == 0 ? m[0] : w == 1 ? m[1] : m[2]; }
+// the bits of frames z0 and on, up to 32 of them
+__device__ __forceinline__ unsigned frames_from(const Mask65& m, int z0) {
+    return z0 < 64 ? (unsigned)(m.lo >> z0) | (z0 > 32 ? m.hi << (64 - z0) : 0u) : m.hi;
+}
 
 // A thread's pixels of a box, tid, tid + blockDim.x, ..., with their column i and row j (stepped, not divided).
 struct PixelWalk {
@@ -408,7 +417,9 @@ __device__ void stage_wait(bool tma, unsigned long long* bar, unsigned parity, f
 constexpr int kClipCand = 1024;     // background voxels above the lowest clip threshold kept per CTA, at most
 constexpr int kFgList = 2048;       // foreground pixels listed per CTA (pass C iterates them densely), at most
 constexpr int kClipWarp = 256;      // candidates that one warp iterates alone
-constexpr int kZBatch = 8;          // voxels of a pixel column loaded together (memory-level parallelism)
+constexpr int kScan = 9;            // voxels of a pixel column that pass 1's scan takes together (depths: 3, 5, 9, 17, ...)
+constexpr int kValid = 17;          // in pass 2, whose scan only compares
+constexpr int kZBatch = 8;          // and pass C, whose frame sums go by eights
 // The gather's threads per row and the frames of a box pixel that a thread reads together. Bound by memory latency
 // (15 of 20 stall cycles) and by how many frames' pages are open at once: more frames in flight a thread make it slower
 // (16 frames: 16.7 ms for the 16M-pixel sweep's 107,446 rows), more pixels of the same frames faster. 128 threads and
@@ -454,7 +465,7 @@ template <int NT> constexpr int min_ctas_pass1() { return 1024 / NT; }
 // with a barrier.
 //
 // Bound by instructions and by the latency of its serial steps, not by bytes: each voxel is read once from DRAM. So
-// the scan of the box (pass A, 40% of a row's time when every voxel took its own tests) takes eight voxels at a time
+// the scan of the box (pass A, 40% of a row's time when every voxel took its own tests) takes nine voxels at a time
 // and tests them together (all valid, none a neighbour's, none above the lowest clip threshold); only a batch that
 // fails goes voxel by voxel. The set-up steps share barriers, the clipping iterations run in one warp, and the
 // per-frame sums of pass C reduce eight frames at a time (warp_sum8).
@@ -464,8 +475,8 @@ template <int NT> constexpr int min_ctas_pass1() { return 1024 / NT; }
 // waits for instructions. Rare branches are rolled, and what a row runs twice is one function. (Loads of the next
 // batch ahead of the tests, in more registers, lost more by their code than they hid: 13.9 ms for the sweep below.)
 //
-// Before and after: 107,446 rows of the 16M-pixel geometry (90 frames, 2.6e9 voxels) 14.2 -> 11.9 ms, 4,096 boxes of
-// 31 x 31 x 33 0.83 -> 0.54 ms, 40,001 of 9 x 9 x 5 0.90 -> 0.63 ms.
+// Before and after: 107,446 rows of the 16M-pixel geometry (90 frames, 2.6e9 voxels) 14.2 -> 11.7 ms, 4,096 boxes of
+// 31 x 31 x 33 0.83 -> 0.54 ms, 40,001 of 9 x 9 x 5 0.90 -> 0.57 ms.
 template <int NT, bool STAGED>
 __device__ __forceinline__ void pass1_row(const XiDetector& det_g, const XiRows& R, const XiBlock& B,
                                           const float* __restrict__ arena, const XiPass1Out& O, int row, int max_bx,
@@ -567,7 +578,7 @@ __device__ __forceinline__ void pass1_row(const XiDetector& det_g, const XiRows&
         fcol[z] = make_float4(frame_centre(iz0, fb, z), e3, e3 * e3, 0.0f);
     }
     const int nact = nb.nact;
-    if (nact) neighbour_axes(R, row, Dz, bx, xs, ys, iz0, fb, nb, tb);
+    if (nact) neighbour_axes(Dz, bx, xs, ys, iz0, fb, nb, tb);
     {
         float e1[3] = {s_e1[0], s_e1[1], s_e1[2]}, e2[3] = {s_e2[0], s_e2[1], s_e2[2]};
         const float Sr[3] = {s_S[0], s_S[1], s_S[2]};
@@ -602,9 +613,9 @@ __device__ __forceinline__ void pass1_row(const XiDetector& det_g, const XiRows&
     // summed again in float64) and its template weight as count * bref, so the float64 totals equal voxel-by-voxel
     // float64 sums.
     const float clip_floor = (0.0f + 3.0f * sqrtf(gain * fmaxf(0.0f, 0.5f))) + 1.0f;
-    const unsigned fgwd[3] = {(unsigned)fgz.lo, (unsigned)(fgz.lo >> 32), fgz.hi};
     {
-        unsigned rec0 = 0u, rec1 = 0u, rec2 = 0u;
+        Mask65 rec;
+        rec.clear();
         int t_over = 0, t_fgm = 0, t_fgnb = 0;
         double a4[4] = {0.0, 0.0, 0.0, 0.0};         // counts, weights; of the voxels no iteration can drop
         PixelWalk px(bx);
@@ -627,66 +638,57 @@ __device__ __forceinline__ void pass1_row(const XiDetector& det_g, const XiRows&
                 bref = bkg_ref(det, xs[px.i], ys[px.j]);
                 brefs[p] = bref;
             }
-            unsigned nbw[3] = {0u, 0u, 0u};
+            Mask65 nbm;
+            nbm.clear();
             if (nact) {
-                const Mask65 m = neighbour_frames(nb, tb, px.i, px.j, Dz);
-                nblo[p] = m.lo;
-                nbw[0] = (unsigned)m.lo;
-                nbw[1] = (unsigned)(m.lo >> 32);
-                nbw[2] = m.hi & 1u;
-                if (nbw[2]) atomicOr(&nbhi[p >> 5], 1u << (p & 31));
+                nbm = neighbour_frames(nb, tb, px.i, px.j, Dz);
+                nblo[p] = nbm.lo;
+                if (nbm.hi) atomicOr(&nbhi[p >> 5], 1u << (p & 31));
             }
             float cs = 0.0f, cs0 = 0.0f, ic = 0.0f;
             int cn = 0, cn0 = 0, in_ = 0;
             bool okall = true;
             const float* col = box + p;
 #pragma unroll 1
-            for (int w = 0; 32 * w < Dz; ++w) {
-                const int zn = min(32, Dz - 32 * w);
-                const unsigned fw = pick3(fgwd, w), nw = pick3(nbw, w);
-                // per voxel only its value's tests are taken (valid, recorded, overloaded bits) and the two sums it
-                // may join; the counts follow from the word's bit masks
-                unsigned vm = 0u, rm = 0u, om = 0u;
-#pragma unroll 1
-                for (int t0 = 0; t0 < zn; t0 += kZBatch, col += (size_t)kZBatch * P) {
-                    const int nbat = min(kZBatch, zn - t0);
-                    const unsigned ib = fw >> t0;          // the batch's foreground frames (the same in every thread)
-                    const unsigned kb = nw >> t0;          // and its neighbours' frames
-                    float v[kZBatch];
+            for (int z0 = 0; z0 < Dz; z0 += kScan, col += (size_t)kScan * P) {
+                const int nbat = min(kScan, Dz - z0);
+                const unsigned all = (1u << nbat) - 1u;
+                const unsigned ib = frames_from(fgz, z0) & all;   // its foreground frames (the same in every thread)
+                const unsigned kb = frames_from(nbm, z0) & all;   // and its neighbours' frames
+                float v[kScan];                            // independent loads in flight before any is used
 #pragma unroll
-                    for (int u = 0; u < kZBatch; ++u) v[u] = u < nbat ? col[(size_t)u * P] : bias;
-                    bool ok = nbat == kZBatch, low = true;
+                for (int u = 0; u < kScan; ++u) v[u] = u < nbat ? col[(size_t)u * P] : bias;
+                bool ok = true, low = true;
 #pragma unroll
-                    for (int u = 0; u < kZBatch; ++u) {
-                        v[u] = v[u] - bias;
-                        ok = ok && v[u] >= 0.0f;
-                        low = low && v[u] <= clip_floor;
+                for (int u = 0; u < kScan; ++u) {
+                    v[u] = v[u] - bias;
+                    ok = ok && v[u] >= 0.0f;
+                    low = low && v[u] <= clip_floor;
+                }
+                unsigned vm = all, rm = all, om = 0u;      // valid, recorded, overloaded
+                if (ok && (low || !ring)) {
+                    if (ib) {
+                        const unsigned m = ib & ~kb;
+#pragma unroll
+                        for (int u = 0; u < kScan; ++u)
+                            if ((m >> u) & 1u) ic += v[u];
                     }
-                    if (ok && (low || !ring)) {
-                        vm |= 0xffu << t0;
-                        rm |= 0xffu << t0;
-                        if (ib & 0xffu) {
-                            const unsigned m = ib & ~kb;
+                    if (ring) {
 #pragma unroll
-                            for (int u = 0; u < kZBatch; ++u)
-                                if ((m >> u) & 1u) ic += v[u];
-                        }
-                        if (ring) {
-#pragma unroll
-                            for (int u = 0; u < kZBatch; ++u)
-                                if (!((kb >> u) & 1u)) cs0 += v[u];
-                            cn0 += __popc(~kb & 0xffu);
-                        }
-                        continue;
+                        for (int u = 0; u < kScan; ++u)
+                            if (!((kb >> u) & 1u)) cs0 += v[u];
+                        cn0 += __popc(all & ~kb);
                     }
+                } else {
+                    vm = rm = 0u;
 #pragma unroll 1
                     for (int u = 0; u < nbat; ++u) {       // voxel by voxel (read again: the batch is near)
                         const float x = col[(size_t)u * P] - bias;
                         const bool valid = x >= 0.0f;
                         const bool mine = valid && !((kb >> u) & 1u);
-                        vm |= (unsigned)valid << (t0 + u);
-                        rm |= (unsigned)(x > -2.5f) << (t0 + u);
-                        om |= (unsigned)(x == -2.0f) << (t0 + u);
+                        vm |= (unsigned)valid << u;
+                        rm |= (unsigned)(x > -2.5f) << u;
+                        om |= (unsigned)(x == -2.0f) << u;
                         if (mine && ((ib >> u) & 1u)) ic += x;
                         if (mine && ring) {                // background (the ring excludes the foreground ellipse)
                             if (x <= clip_floor) {
@@ -706,24 +708,23 @@ __device__ __forceinline__ void pass1_row(const XiDetector& det_g, const XiRows&
                         }
                     }
                 }
-                if (w == 0) rec0 |= rm;
-                else if (w == 1) rec1 |= rm;
-                else rec2 |= rm;
-                const unsigned fgm = fg2 ? fw : 0u;     // foreground voxels of this column
+                if (z0 < 64) rec.lo |= (unsigned long long)rm << z0;
+                if (z0 > 64 - kScan) rec.hi |= z0 < 64 ? rm >> (64 - z0) : rm;
+                if (!ib) continue;
+                const unsigned fgm = fg2 ? ib : 0u;       // foreground voxels of the batch
                 t_over += __popc(fgm & om);
                 t_fgm += __popc(fgm & ~vm & rm);
-                t_fgnb += __popc(fgm & nw);
-                const unsigned clean_fg = fw & vm & ~nw; // foreground-frame voxels valid and not a neighbour's
+                t_fgnb += __popc(fgm & kb);
+                const unsigned clean_fg = ib & vm & ~kb;   // foreground-frame voxels valid and not a neighbour's
                 in_ += __popc(clean_fg);
-                if (clean_fg != fw) okall = false;
+                if (clean_fg != ib) okall = false;
             }
             double csd = (double)cs;
             if (cs >= 16777216.0f) {                     // float32 may have rounded: this column again in float64
                 csd = 0.0;
                 for (int z = 0; z < Dz; ++z) {
                     const float v = box[(size_t)z * P + p] - bias;
-                    const bool nbz = (pick3(nbw, z >> 5) >> (z & 31)) & 1u;
-                    if (ring && v >= 0.0f && !nbz && v > clip_floor) csd += (double)v;
+                    if (ring && v >= 0.0f && !nbm.get(z) && v > clip_floor) csd += (double)v;
                 }
             }
             a4[0] += csd + (double)cs0;
@@ -733,7 +734,7 @@ __device__ __forceinline__ void pass1_row(const XiDetector& det_g, const XiRows&
             ics[p] = ic;                                 // completed with the background after pass B
             imgn[p] = (unsigned char)(in_ | (okall ? 0x80 : 0));
         }
-        const unsigned r3[3] = {rec0, rec1, rec2};
+        const unsigned r3[3] = {(unsigned)rec.lo, (unsigned)(rec.lo >> 32), rec.hi};
 #pragma unroll
         for (int w = 0; w < 3; ++w) {
             const unsigned r = __reduce_or_sync(0xffffffffu, r3[w]);
@@ -874,16 +875,15 @@ __device__ __forceinline__ void pass1_row(const XiDetector& det_g, const XiRows&
         }
         if (!__any_sync(0xffffffffu, have)) continue;      // warp-uniform: no foreground pixel in this warp
         float u1 = 0.f, u2 = 0.f, bref = 1.f;
-        unsigned nbw[3] = {0u, 0u, 0u};
+        Mask65 nbm;
+        nbm.clear();
         if (have) {
             u1 = O.u1[po + p];
             u2 = O.u2[po + p];
             if (templ) bref = brefs[p];
             if (nact) {
-                const unsigned long long nl = nblo[p];
-                nbw[0] = (unsigned)nl;
-                nbw[1] = (unsigned)(nl >> 32);
-                if (max_dz > 64) nbw[2] = (nbhi[p >> 5] >> (p & 31)) & 1u;
+                nbm.lo = nblo[p];
+                if (max_dz > 64) nbm.hi = (nbhi[p >> 5] >> (p & 31)) & 1u;
             }
         }
         const float bpix = b * bref;
@@ -893,7 +893,7 @@ __device__ __forceinline__ void pass1_row(const XiDetector& det_g, const XiRows&
 #pragma unroll 1
         for (int z0 = 0; z0 < Dz; z0 += kZBatch, col += (size_t)kZBatch * P) {
             const int nbat = min(kZBatch, Dz - z0);
-            const unsigned ib = pick3(fgwd, z0 >> 5) >> (z0 & 31), kb = pick3(nbw, z0 >> 5) >> (z0 & 31);
+            const unsigned ib = frames_from(fgz, z0), kb = frames_from(nbm, z0);
             float v[kZBatch];
 #pragma unroll
             for (int u = 0; u < kZBatch; ++u) v[u] = have && u < nbat ? col[(size_t)u * P] : 0.0f;
@@ -1117,16 +1117,16 @@ __device__ __forceinline__ void group_sum(double (&v)[NV], unsigned which, int n
 //
 // Bound by instructions and by the latency of its serial steps, as pass 1. Only a few percent of a box's voxels enter
 // the fit, those where the profile exceeds a hundredth of its largest value, while every voxel's validity counts (for
-// the profile share on valid voxels). So the scan of the box tests validity alone (a compare a voxel, eight loads in
-// flight), and the pixels whose column can hold fitted voxels are listed and taken again, a thread a run of up to
+// the profile share on valid voxels). So the scan of the box tests validity alone (a compare a voxel, 17 loads in
+// flight: 10.3 ms for the sweep below, 10.8 with nine), and the pixels whose column can hold fitted voxels are listed and taken again, a thread a run of up to
 // nine frames. Six rounds of the fit then run on the compacted fitted voxels in few warps, with one barrier a round
 // (none for one warp) and only the sums the row needs; the other warps are done.
 // Where the list overflows, the runs that did not fit are taken from the box again in every round (the rows used to
 // scan their whole box).
 //
-// Before and after: 107,446 rows of the 16M-pixel geometry (90 frames, 500 fitted voxels a row) 17.0 -> 11.5 ms, 4,096
-// boxes of 31 x 31 x 33 (5,350 fitted) 2.89 -> 1.07 ms, 1,003 of 41 x 41 x 65 (21,000 fitted) 6.86 -> 2.29 ms, 40,001 of
-// 9 x 9 x 5 1.29 -> 0.86 ms.
+// Before and after: 107,446 rows of the 16M-pixel geometry (90 frames, 500 fitted voxels a row) 17.0 -> 9.3 ms, 4,096
+// boxes of 31 x 31 x 33 (5,350 fitted) 2.89 -> 1.05 ms, 1,003 of 41 x 41 x 65 (21,000 fitted) 6.86 -> 1.36 ms, 40,001 of
+// 9 x 9 x 5 1.29 -> 0.89 ms.
 template <int NT, bool STAGED>
 __device__ __forceinline__ void pass2_row(const XiDetector& det_g, const XiRows& R, const XiBlock& B,
                                           const float* __restrict__ arena, const float* __restrict__ prof,
@@ -1223,7 +1223,7 @@ __device__ __forceinline__ void pass2_row(const XiDetector& det_g, const XiRows&
         if (!has_p) fRp[z] = 0.0f;
     }
     const int nact = nb.nact;
-    if (nact) neighbour_axes(R, row, Dz, bx, xs, ys, iz0, fb, nb, tb);
+    if (nact) neighbour_axes(Dz, bx, xs, ys, iz0, fb, nb, tb);
     if (has_p) {
         float e1[3] = {s_e1[0], s_e1[1], s_e1[2]}, e2[3] = {s_e2[0], s_e2[1], s_e2[2]};
         float S[3] = {s_S[0], s_S[1], s_S[2]};
@@ -1310,30 +1310,28 @@ __device__ __forceinline__ void pass2_row(const XiDetector& det_g, const XiRows&
                     may = may || (P2p * Rpmax) * hp > ppthr || P2p < 0.0f;
                 }
                 if (templ) brefs[p] = bkg_ref(det, xs[px.i], ys[px.j]);
-                unsigned nbw[3] = {0u, 0u, 0u};
+                Mask65 nbm;
+                nbm.clear();
                 if (nact) {
-                    const Mask65 m = neighbour_frames(nb, tb, px.i, px.j, Dz);
-                    nblo[p] = m.lo;
-                    nbw[0] = (unsigned)m.lo;
-                    nbw[1] = (unsigned)(m.lo >> 32);
-                    nbw[2] = m.hi & 1u;
-                    if (nbw[2]) atomicOr(&nbhi[p >> 5], 1u << (p & 31));
+                    nbm = neighbour_frames(nb, tb, px.i, px.j, Dz);
+                    nblo[p] = nbm.lo;
+                    if (nbm.hi) atomicOr(&nbhi[p >> 5], 1u << (p & 31));
                 }
                 float lost = 0.0f;                   // rocking-curve weight of the frames this pixel loses
                 const float* col = box + p;
-                for (int t0 = 0; t0 < Dz; t0 += kZBatch, col += (size_t)kZBatch * P) {
-                    const int nbat = min(kZBatch, Dz - t0);
-                    const unsigned kb = pick3(nbw, t0 >> 5) >> (t0 & 31);
-                    float v[kZBatch];
+                for (int z0 = 0; z0 < Dz; z0 += kValid, col += (size_t)kValid * P) {
+                    const int nbat = min(kValid, Dz - z0);
+                    const unsigned kb = frames_from(nbm, z0) & ((1u << nbat) - 1u);
+                    float v[kValid];
 #pragma unroll
-                    for (int u = 0; u < kZBatch; ++u) v[u] = u < nbat ? col[(size_t)u * P] : bias;
-                    bool ok = (kb & 0xffu) == 0u;
+                    for (int u = 0; u < kValid; ++u) v[u] = u < nbat ? col[(size_t)u * P] : bias;
+                    bool ok = kb == 0u;
 #pragma unroll
-                    for (int u = 0; u < kZBatch; ++u) ok = ok && v[u] >= bias;      // value >= 0
+                    for (int u = 0; u < kValid; ++u) ok = ok && v[u] >= bias;      // value >= 0
                     if (ok) continue;
 #pragma unroll
-                    for (int u = 0; u < kZBatch; ++u)
-                        if (u < nbat && !(v[u] >= bias && !((kb >> u) & 1u))) lost += fR[t0 + u];
+                    for (int u = 0; u < kValid; ++u)
+                        if (u < nbat && !(v[u] >= bias && !((kb >> u) & 1u))) lost += fR[z0 + u];
                 }
                 const double tp = (double)P2 * r_all;
                 a8[2] += tp;
@@ -1960,7 +1958,7 @@ constexpr size_t kPass2Share = 69 * 1024;
 // Launch tuning (xi_tune): the largest shoebox each pass stages in shared memory, and the fit-list capacity of
 // pass 2. Larger staging overlaps the box read with the set-up but costs resident CTAs per SM.
 size_t g_stage_max[2] = {48 * 1024, 48 * 1024};
-int g_list_cap[2] = {2048, 8192};   // boxes up to XI_PASS2_LARGE_VOXELS voxels, larger boxes
+int g_list_cap[2] = {2048, 2048};   // boxes up to XI_PASS2_LARGE_VOXELS voxels, larger boxes (at least: pass2_plan)
 int g_wide_nt = 256;          // threads per CTA of the pass kernels for boxes over 200 pixels (128 or 256)
 
 // Pass 1 stages boxes of up to g_stage_max[0] bytes when they fit beside the per-pixel tables.
@@ -1973,10 +1971,11 @@ bool pass1_staged(int max_bx, int max_dz, int K) {
 // the box is staged, and the fit's lists. The largest boxes (up to 97 px, 65 frames) take what the device allows a CTA
 // beyond the kernel's static arrays, not the default budget. The list of fitted voxels holds up to every voxel of small
 // boxes, and of large ones g_list_cap voxels (the second capacity for launches whose largest box exceeds
-// XI_PASS2_LARGE_VOXELS voxels or XI_PASS2_LARGE_DEPTH bins: a deep rocking curve keeps many frames above the profile
-// threshold, and fewer CTAs per SM pay less there) or, where that is more, what a third of an SM's shared memory
-// leaves it (4,096 boxes of 31 x 31 x 33 with 5,350 fitted voxels a box: 1.07 ms in place of 1.36 with a list for 40 KB
-// a CTA and 1.13 with one for 100 KB, which costs the 16M-pixel sweep 3 ms of 11.5 for the CTAs lost). Runs that do not
+// XI_PASS2_LARGE_VOXELS voxels or XI_PASS2_LARGE_DEPTH bins) or, where that is more, what a third of an SM's shared
+// memory leaves it: 4,096 boxes of 31 x 31 x 33 with 5,350 fitted voxels a box take 1.07 ms so, 1.36 with a list for
+// 40 KB a CTA and 1.13 with one for 100 KB, which costs the 16M-pixel sweep 3 ms for the CTAs lost. (8,192 voxels for
+// the larger boxes, the choice while rows scanned their box when the list overflowed, left two CTAs an SM there: 2.15 ms
+// for 1,003 boxes of 41 x 41 x 65, 1.36 with the third; the sweep's pass 2 10.3 and 9.3 ms.) Runs that do not
 // fit are taken from the box in every round. The box is staged only when small (it is read once: staging buys the
 // copy's overlap with the set-up, not re-reads).
 int pass2_plan(int max_bx, int max_dz, int K, const char* who, bool* staged, Fit* fit) {

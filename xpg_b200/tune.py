@@ -3,8 +3,8 @@
 A batched launch sizes its shared memory, threads per CTA and staging for the largest box of its bin: wide bins
 put small boxes in CTAs sized for large ones (fewer resident CTAs), narrow bins make more launches (more tails). The
 CTA shape of large boxes (128 threads at 6 CTAs per SM, or 256 at 3), the largest box staged in shared memory by
-a bulk copy, and pass 2's fit-list capacity (the fitted voxels kept in shared memory for its six IRLS iterations;
-a row with more fits from the box each time) trade resident reflections per SM against work per CTA. The tuner
+a bulk copy, and pass 2's least fit-list capacity (the fitted voxels kept in shared memory for its six IRLS iterations;
+the rest comes from the box each time) trade resident reflections per SM against work per CTA. The tuner
 times pass 1 and pass 2 of real blocks for launch shapes, then list capacities, then candidate bin edges (subsets of
 the box-side buckets present, at most `max_bins` bins), and keeps the fastest; results are stored per device name in `tuned.json` beside this file, which the library applies
 when it loads (`native.load`) and `device.batched_items` reads.
@@ -56,7 +56,7 @@ SHAPES = ({"wide_threads": 256, "pass1_stage_bytes": 48 * 1024}, {"wide_threads"
 
 
 LIST_CAPS = (2048, 4096, 8192, 12288, 16384)
-CAP_DEFAULTS = {"pass2_list_cap": 2048, "pass2_list_cap_large": 8192}
+CAP_DEFAULTS = {"pass2_list_cap": 2048, "pass2_list_cap_large": 2048}
 
 
 def _apply(shape):
