@@ -30,11 +30,28 @@ def _np(v):
     return np.asarray(v)
 
 
+# the tensors that have a numpy form; the others (bfloat16, float8, views with a pending conjugate or sign) are refused
+_TYPES = frozenset((torch.float64, torch.float32, torch.float16, torch.int64, torch.int32, torch.int16, torch.int8,
+                    torch.uint64, torch.uint32, torch.uint16, torch.uint8, torch.bool, torch.complex64,
+                    torch.complex128))
+
+
 def _in(v):
     """A per-row or per-pixel argument for `device._dev`: a CUDA tensor as it is (it is converted on the device, or
     read in place), anything else as a numpy array. Through the host instead, the pixel tables' copies alone took
     most of a call (4096 boxes of 31 x 31 x 33: 26.3 ms for the three passes, 3.8 ms of it kernels)."""
-    return v.detach() if torch.is_tensor(v) and v.is_cuda else _np(v)
+    if not (torch.is_tensor(v) and v.is_cuda):
+        return _np(v)
+    if v.dtype not in _TYPES or v.is_neg() or v.is_conj():
+        raise TypeError(f"argument of type {v.dtype}" + (" with a pending sign or conjugate" if v.dtype in _TYPES else "")
+                        + " has no numpy form")
+    return v.detach()
+
+
+def _as(v, dtype):
+    """`_in`, a numpy array converted to `dtype` by numpy (which takes foreign byte orders and long doubles)."""
+    v = _in(v)
+    return v if torch.is_tensor(v) else v.astype(dtype)
 
 
 def _on_device(v):
@@ -46,7 +63,7 @@ def _on_device(v):
 def _rows(sb, rc, nb, Dz, Dx):
     n = int(sb.shape[0])
     one = ("S", "phi", "ix0", "iy0", "iz0", "fb", "region", "has_p", "pS", "pphi")
-    pxs = _in(rc["pxs"]) if "pxs" in rc else np.ones(n, np.int32)
+    pxs = _as(rc["pxs"], np.int32) if "pxs" in rc else np.ones(n, np.int32)
     return D.RowSet(**{k: _in(rc[k]) for k in one}, pxs=pxs, Dz=np.full(n, Dz), bx=np.full(n, Dx),
                     nb={k: _in(nb[k]) for k in ("x", "y", "z", "sx", "sz")}, sb_bias=0.0)
 
@@ -139,7 +156,7 @@ def make_kernels(Dz, Dy, Dx, n_regions, G=PROFILE_GRID):
             buf.t[k].copy_(_on_device(v).reshape(-1).float())
         blk, keep = _block(axis, s0, frames_phi0, osc, sd, sm, gain, rcw)
         out = D.Pass2Buffers(rows)
-        proft = _on_device(prof).float().contiguous()
+        proft = _on_device(_as(prof, np.float32)).float().contiguous()
         D.pass2(det, rows, blk, arena, proft, buf, out, groups=_groups(rows))
         D.status()
         return dict(out.t)
