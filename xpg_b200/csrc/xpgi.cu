@@ -430,12 +430,12 @@ constexpr int kGatherBatch = 4;
 
 // Dynamic shared memory of pass 1 for boxes up to max_bx pixels a side and max_dz bins with K neighbour columns: the
 // neighbours' frame masks (8P) | geometry scratch eps1, then the background template (4P) | eps2, then the img2 counts
-// (4P) | per pixel the number of clean foreground-frame voxels and the all-clean bit (P) | frame 64's neighbour bits
-// and the foreground pixels (a bit each) | foreground list | rocking-curve terms, then the clip candidates | the
+// (4P) | per pixel the number of clean foreground-frame voxels and the all-clean bit (P) | frame 64's neighbour bits,
+// the foreground pixels and the background ring's (a bit each) | foreground list | rocking-curve terms, then the clip candidates | the
 // neighbours' axis terms | staged shoebox.
 struct Pass1Layout {
     int Pm, cap, fgcap;
-    size_t e1, e2, imgn, hi, fg, fgl, scr, nbt, stage, bytes;
+    size_t e1, e2, imgn, hi, fg, ring, fgl, scr, nbt, stage, bytes;
 
     __host__ __device__ Pass1Layout(int max_bx, int max_dz, int K, bool staged) {
         Pm = max_bx * max_bx;
@@ -446,7 +446,8 @@ struct Pass1Layout {
         imgn = e2 + (size_t)4 * Pm;
         hi = (imgn + Pm + 3) / 4 * 4;
         fg = hi + (max_dz > 64 ? (size_t)(Pm + 31) / 32 * 4 : 0);
-        fgl = fg + (size_t)(Pm + 31) / 32 * 4;
+        ring = fg + (size_t)(Pm + 31) / 32 * 4;
+        fgl = ring + (size_t)(Pm + 31) / 32 * 4;
         scr = (fgl + (size_t)2 * fgcap + 15) / 16 * 16;
         const size_t c = (size_t)6 * cap, t = (size_t)max_dz * XI_RC_K * sizeof(float);
         nbt = (scr + (c > t ? c : t) + 15) / 16 * 16;
@@ -466,17 +467,20 @@ template <int NT> constexpr int min_ctas_pass1() { return 1024 / NT; }
 //
 // Bound by instructions and by the latency of its serial steps, not by bytes: each voxel is read once from DRAM. So
 // the scan of the box (pass A, 40% of a row's time when every voxel took its own tests) takes nine voxels at a time
-// and tests them together (all valid, none a neighbour's, none above the lowest clip threshold); only a batch that
-// fails goes voxel by voxel. The set-up steps share barriers, the clipping iterations run in one warp, and the
+// and tests them together (all valid, none above the lowest clip threshold): a batch that passes needs only its sums,
+// one that fails makes its masks and splits its sums by them, from the same registers. Going voxel by voxel through such
+// a batch, its values read again, was 1.25 times the time of one loop over all voxels where the background lies above
+// the threshold (1,261 boxes of 31 x 31 x 33 with 20 counts a voxel: 0.527 ms, 0.662 so, 0.517 now), and most columns of
+// a common box hold such a batch. The set-up steps share barriers, the clipping iterations run in one warp, and the
 // per-frame sums of pass C reduce eight frames at a time (warp_sum8).
 //
-// Code size counts: the resident CTAs' warps are in different steps of a row, and with the loops over 32-frame words,
-// the voxel-by-voxel branch and the error functions unrolled or inlined several times, a third of the stalls were
-// waits for instructions. Rare branches are rolled, and what a row runs twice is one function. (Loads of the next
-// batch ahead of the tests, in more registers, lost more by their code than they hid: 13.9 ms for the sweep below.)
+// Code size counts: the resident CTAs' warps are in different steps of a row, and with the loops over 32-frame words
+// and the error functions unrolled or inlined several times, a third of the stalls were waits for instructions. What a
+// row runs twice is one function. (Loads of the next batch ahead of the tests, in more registers, lost more by their
+// code than they hid: 13.9 ms in place of 12.1 for the sweep below at that stage.)
 //
-// Before and after: 107,446 rows of the 16M-pixel geometry (90 frames, 2.6e9 voxels) 14.2 -> 11.7 ms, 4,096 boxes of
-// 31 x 31 x 33 0.83 -> 0.54 ms, 40,001 of 9 x 9 x 5 0.90 -> 0.57 ms.
+// Before and after: 107,446 rows of the 16M-pixel geometry (90 frames, 2.6e9 voxels) 14.2 -> 9.5 ms, 4,096 boxes of
+// 31 x 31 x 33 0.83 -> 0.48 ms, 40,001 of 9 x 9 x 5 0.90 -> 0.52 ms.
 template <int NT, bool STAGED>
 __device__ __forceinline__ void pass1_row(const XiDetector& det_g, const XiRows& R, const XiBlock& B,
                                           const float* __restrict__ arena, const XiPass1Out& O, int row, int max_bx,
@@ -527,6 +531,7 @@ __device__ __forceinline__ void pass1_row(const XiDetector& det_g, const XiRows&
     unsigned char* imgn = dyn1 + L.imgn;            // per pixel: clean foreground-frame voxels | all-clean bit 7
     unsigned* nbhi = reinterpret_cast<unsigned*>(dyn1 + L.hi);
     unsigned* fgw = reinterpret_cast<unsigned*>(dyn1 + L.fg);
+    unsigned* ringw = reinterpret_cast<unsigned*>(dyn1 + L.ring);
     unsigned short* fgl = reinterpret_cast<unsigned short*>(dyn1 + L.fgl);
     float* terms = reinterpret_cast<float*>(dyn1 + L.scr);
     float* cand_v = terms;
@@ -630,8 +635,11 @@ __device__ __forceinline__ void pass1_row(const XiDetector& det_g, const XiRows&
                 fg2 = r2 <= kFgR2;
                 ring = r2 >= kBgR2;
             }
-            const unsigned ball = __ballot_sync(0xffffffffu, fg2);
-            if (lane == 0 && p < P) fgw[p >> 5] = ball;
+            const unsigned ball = __ballot_sync(0xffffffffu, fg2), rball = __ballot_sync(0xffffffffu, ring);
+            if (lane == 0 && p < P) {
+                fgw[p >> 5] = ball;
+                ringw[p >> 5] = rball;
+            }
             if (p >= P) continue;
             float bref = 1.0f;
             if (templ) {
@@ -663,48 +671,55 @@ __device__ __forceinline__ void pass1_row(const XiDetector& det_g, const XiRows&
                 for (int u = 0; u < kScan; ++u) {
                     v[u] = v[u] - bias;
                     ok = ok && v[u] >= 0.0f;
-                    low = low && v[u] <= clip_floor;
+                    low = low && v[u] <= clip_floor;       // (false of NaN)
                 }
                 unsigned vm = all, rm = all, om = 0u;      // valid, recorded, overloaded
-                if (ok && (low || !ring)) {
-                    if (ib) {
-                        const unsigned m = ib & ~kb;
-#pragma unroll
-                        for (int u = 0; u < kScan; ++u)
-                            if ((m >> u) & 1u) ic += v[u];
-                    }
-                    if (ring) {
-#pragma unroll
-                        for (int u = 0; u < kScan; ++u)
-                            if (!((kb >> u) & 1u)) cs0 += v[u];
-                        cn0 += __popc(all & ~kb);
-                    }
-                } else {
+                if (!ok) {
                     vm = rm = 0u;
-#pragma unroll 1
-                    for (int u = 0; u < nbat; ++u) {       // voxel by voxel (read again: the batch is near)
-                        const float x = col[(size_t)u * P] - bias;
-                        const bool valid = x >= 0.0f;
-                        const bool mine = valid && !((kb >> u) & 1u);
-                        vm |= (unsigned)valid << u;
-                        rm |= (unsigned)(x > -2.5f) << u;
-                        om |= (unsigned)(x == -2.0f) << u;
-                        if (mine && ((ib >> u) & 1u)) ic += x;
-                        if (mine && ring) {                // background (the ring excludes the foreground ellipse)
-                            if (x <= clip_floor) {
-                                cs0 += x;
-                                ++cn0;
-                            } else {
-                                cs += x;
-                                ++cn;
-                                if (use_list) {
-                                    const int k = atomicAdd(&s_ncand, 1);
-                                    if (k < L.cap) {
-                                        cand_v[k] = x;
-                                        cand_p[k] = (unsigned short)p;
-                                    }
-                                }
+#pragma unroll
+                    for (int u = 0; u < kScan; ++u) {
+                        vm |= (unsigned)(v[u] >= 0.0f) << u;
+                        rm |= (unsigned)(v[u] > -2.5f) << u;
+                        om |= (unsigned)(v[u] == -2.0f) << u;
+                    }
+                    vm &= all;
+                    rm &= all;
+                }
+                const unsigned mine = vm & ~kb;            // valid and not a neighbour's
+                if (ib) {
+                    const unsigned m = ib & mine;
+#pragma unroll
+                    for (int u = 0; u < kScan; ++u)
+                        if ((m >> u) & 1u) ic += v[u];
+                }
+                if (ring) {                                // background (the ring excludes the foreground ellipse)
+                    unsigned hm = 0u;                      // its voxels above the lowest clip threshold
+                    if (low) {
+#pragma unroll
+                        for (int u = 0; u < kScan; ++u)
+                            if ((mine >> u) & 1u) cs0 += v[u];
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < kScan; ++u)
+                            if ((mine >> u) & 1u) {
+                                const bool up = !(v[u] <= clip_floor);
+                                hm |= (unsigned)up << u;
+                                cs0 += up ? 0.0f : v[u];
+                                cs += up ? v[u] : 0.0f;
                             }
+                    }
+                    cn0 += __popc(mine & ~hm);
+                    if (hm) {
+                        cn += __popc(hm);
+                        // listed while the list has room (a full list is not used, so it need not be counted on)
+                        if (use_list && *(volatile int*)&s_ncand <= L.cap) {
+                            int k = atomicAdd(&s_ncand, __popc(hm));
+#pragma unroll 1
+                            for (unsigned r = hm; r; r &= r - 1u, ++k)
+                                if (k < L.cap) {           // (the value read again: the batch is near)
+                                    cand_v[k] = col[(size_t)(__ffs(r) - 1) * P] - bias;
+                                    cand_p[k] = (unsigned short)p;
+                                }
                         }
                     }
                 }
@@ -822,8 +837,7 @@ __device__ __forceinline__ void pass1_row(const XiDetector& det_g, const XiRows&
                 clip_candidates(threadIdx.x, NT, a2[0], a2[1]);
             } else {
                 for (int p = threadIdx.x; p < P; p += NT) {
-                    const float u1 = O.u1[po + p], u2 = O.u2[po + p];
-                    if (!(u1 * u1 + u2 * u2 >= kBgR2)) continue;      // also excludes the foreground ellipse
+                    if (!((ringw[p >> 5] >> (p & 31)) & 1u)) continue;
                     const float bref = templ ? brefs[p] : 1.0f;
                     const float thr = clip_threshold(b * bref);
                     Mask65 nbm;
