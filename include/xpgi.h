@@ -153,10 +153,10 @@ int xi_status(void *stream);
 int xi_status_copy(int *host_dst, void *stream);
 
 /* Launch tuning (process-wide; no counterpart in XPG, whose torch kernels have no launch shape): the largest
- * shoebox (bytes) pass 1 / pass 2 stage in shared memory, pass 2's least fit-list capacity (voxels; 256-thread CTAs
- * take what a third of an SM leaves, 0: no list) for launches whose largest box is up to XI_PASS2_LARGE_VOXELS voxels
- * and XI_PASS2_LARGE_DEPTH bins deep and for larger ones, and the CTA width of large boxes. Results do not depend on
- * these. */
+ * shoebox (bytes) pass 1 / pass 2 stage in shared memory (pass 2 only where that costs no CTA an SM), pass 2's least
+ * fit-list capacity (voxels; as many CTAs share an SM as hold such a list, and the list takes what their share leaves;
+ * 0: no list) for launches whose largest box is up to XI_PASS2_LARGE_VOXELS voxels and XI_PASS2_LARGE_DEPTH bins deep
+ * and for larger ones, and the CTA width of large boxes. Results do not depend on these. */
 #define XI_TUNE_PASS1_STAGE_BYTES 1
 #define XI_TUNE_PASS2_STAGE_BYTES 2
 #define XI_TUNE_PASS2_LIST_CAP 3

@@ -1,5 +1,7 @@
-"""Pass 1 and pass 2 where a box's values take them off their common path: backgrounds that all lie above the lowest clip
-threshold (the list of clip candidates overflows), scattered masked voxels, NaN voxels (not valid, not recorded). Against the oracle: masks, counts, background and per-pixel terms bit for bit, sums within 1e-5 of their scale."""
+"""Pass 1 and pass 2 where a box's values or its spot take them off their common path: backgrounds that all lie above the
+lowest clip threshold (the list of clip candidates overflows), scattered masked voxels, NaN voxels (not valid, not
+recorded), and spots so wide that the fitted voxels overflow their list, with the candidate pixels inside or beyond
+theirs. Against the oracle: masks, counts, background and per-pixel terms bit for bit, sums within 1e-5 of their scale."""
 from __future__ import annotations
 
 import numpy as np
@@ -71,3 +73,31 @@ def test_bright_masked_and_nan_boxes(case, bx, Dz, stage, tuned):
     sb[2][rng.random(sb.shape[1:]) < 0.3] = -1.0
     sb[3][rng.random(sb.shape[1:]) < 0.03] = np.nan
     _compare((case, bx, Dz), _run(case, d, sb, one, nb))
+
+
+@pytest.mark.parametrize("wide,cap", [(256, 2048), (256, 0), (128, 2048)])
+@pytest.mark.parametrize("bx,Dz,pixels,voxels", [(31, 33, 0, 7000), (41, 65, 0, 20000), (73, 17, 2048, 20000),
+                                                 (97, 1, 2048, 4000), (97, 65, 2048, 50000)])
+def test_wide_spots(bx, Dz, pixels, voxels, wide, cap, tuned):
+    """Spots that fill their boxes: more fitted voxels than any list of the shape holds, and of 97 px boxes more
+    candidate pixels than the pixel list."""
+    from xpg_b200 import native as N
+    tuned(N.XI_TUNE_WIDE_THREADS, wide)
+    tuned(N.XI_TUNE_PASS2_LIST_CAP, cap)
+    tuned(N.XI_TUNE_PASS2_LIST_CAP_LARGE, cap)
+    d, sb, one, nb = _rows("crowded", bx, Dz, 3, bx + Dz)
+    one["has_p"] = np.array([1.0, 0.0, 1.0], np.float32) * (one["has_p"] > 0.5)
+    nb = {k: v.copy() for k, v in nb.items()}
+    for k in ("sx", "sz"):
+        nb[k][:2] *= np.float32(0.01)                      # (neighbours of the third row only)
+    spec, tmpl, _, _ = G.case_inputs("crowded")
+    odet = OK.detector_consts(spec.geometry(), tmpl)
+    r = G.row_dict(one, 0)
+    gt = OK.geometry(odet, r, (Dz, bx, bx), d["s0"], d["axis"], d["frames_phi0"], d["osc"], d["sd"], d["sm"], d["rcw"])
+    widen = abs(float(gt["u1"][bx // 2, 0])) / 2.2
+    sm = abs(float(gt["zeta"])) * float(d["osc"]) * max(Dz, 3) / 6.0
+    gt = OK.geometry(odet, r, (Dz, bx, bx), d["s0"], d["axis"], d["frames_phi0"], d["osc"], d["sd"] * widen, sm, d["rcw"])
+    plane = OK.profile_plane(d["prof"][int(r["region"])], gt)
+    p = plane[None] * gt["R"][:, None, None]
+    assert (p > 0.01 * p.max()).sum() > voxels and (p.max(0) > 0.01 * p.max()).sum() > pixels
+    _compare((bx, Dz, wide, cap), _run("crowded", d, sb, one, nb, widen, sm))

@@ -1070,7 +1070,7 @@ __global__ void __launch_bounds__(NT, min_ctas_pass1<NT>()) k_pass1_q(const XiRo
 // ==================================================================================================================
 // pass 2
 // ==================================================================================================================
-constexpr int kFitPix = 2048;       // pixels that may hold fitted voxels, listed per CTA, at most
+constexpr int kFitPix = 2048;       // pixels that may hold fitted voxels, listed per CTA, when not all of the box's can be
 constexpr int kFitChunk = 9;        // frames of such a pixel that a thread takes
 constexpr int kFitWarp = 128;       // listed voxels that a warp of the fit takes
 
@@ -1965,14 +1965,16 @@ int launch_pass2_q(const XiRowSet* sets, const int64_t* items, int n_items, int 
 // Dynamic shared memory available beside the kernels' static arrays (bytes).
 constexpr size_t kStageBudget = 190 * 1024;
 
-// Dynamic shared memory a pass-2 CTA of 256 threads may use when three share an SM (228 KB; 1 KB and the static arrays,
-// under 5 KB, go off each share).
-constexpr size_t kPass2Share = 69 * 1024;
+// Dynamic shared memory of a pass-2 CTA of nt threads when n share an SM: 228 KB an SM, of which each CTA loses 1 KB and
+// its static arrays (at most 4,032 bytes of 64 threads, 4,304 of 128, 4,848 of 256).
+constexpr size_t pass2_share(int n, int nt) {
+    return (size_t)228 * 1024 / n - 1024 - (nt == 64 ? 4096 : nt == 128 ? 4352 : 4864);
+}
 
 // Launch tuning (xi_tune): the largest shoebox each pass stages in shared memory, and the fit-list capacity of
 // pass 2. Larger staging overlaps the box read with the set-up but costs resident CTAs per SM.
 size_t g_stage_max[2] = {48 * 1024, 48 * 1024};
-int g_list_cap[2] = {2048, 2048};   // boxes up to XI_PASS2_LARGE_VOXELS voxels, larger boxes (at least: pass2_plan)
+int g_list_cap[2] = {2048, 2048};   // boxes up to XI_PASS2_LARGE_VOXELS voxels, larger boxes: the least list (pass2_plan)
 int g_wide_nt = 256;          // threads per CTA of the pass kernels for boxes over 200 pixels (128 or 256)
 
 // Pass 1 stages boxes of up to g_stage_max[0] bytes when they fit beside the per-pixel tables.
@@ -1981,52 +1983,52 @@ bool pass1_staged(int max_bx, int max_dz, int K) {
            Pass1Layout(max_bx, max_dz, K, true).bytes <= kStageBudget;
 }
 
+// threads of a pass CTA for boxes up to max_bx pixels a side
+int pass_threads(int max_bx) {
+    const int P = max_bx * max_bx;
+    return P <= 96 ? 64 : P <= 200 || g_wide_nt == 128 ? 128 : 256;
+}
+
 // Pass 2's shared-memory plan for boxes up to max_bx pixels a side and max_dz bins with K neighbour columns: whether
-// the box is staged, and the fit's lists. The largest boxes (up to 97 px, 65 frames) take what the device allows a CTA
-// beyond the kernel's static arrays, not the default budget. The list of fitted voxels holds up to every voxel of small
-// boxes, and of large ones g_list_cap voxels (the second capacity for launches whose largest box exceeds
-// XI_PASS2_LARGE_VOXELS voxels or XI_PASS2_LARGE_DEPTH bins) or, where that is more, what a third of an SM's shared
-// memory leaves it: 4,096 boxes of 31 x 31 x 33 with 5,350 fitted voxels a box take 1.07 ms so, 1.36 with a list for
-// 40 KB a CTA and 1.13 with one for 100 KB, which costs the 16M-pixel sweep 3 ms for the CTAs lost. (8,192 voxels for
-// the larger boxes, the choice while rows scanned their box when the list overflowed, left two CTAs an SM there: 2.15 ms
-// for 1,003 boxes of 41 x 41 x 65, 1.36 with the third; the sweep's pass 2 10.3 and 9.3 ms.) Runs that do not
-// fit are taken from the box in every round. The box is staged only when small (it is read once: staging buys the
-// copy's overlap with the set-up, not re-reads).
-int pass2_plan(int max_bx, int max_dz, int K, const char* who, bool* staged, Fit* fit) {
+// the box is staged, and the fit's lists. First the CTAs that an SM holds: as many as the registers allow, fewer where
+// the tables with the least list (g_list_cap voxels, or the whole box) need more room than their share. Then what that
+// share leaves goes to the box, staged where it is small and costs no CTA, to the list of pixels (all of the box's where
+// the least list still fits, else kFitPix) and to the list of voxels. Runs that
+// do not fit the list are taken from the box in every round; the second least list is for launches whose largest box
+// exceeds XI_PASS2_LARGE_VOXELS voxels or XI_PASS2_LARGE_DEPTH bins; 0 voxels: no list.
+// A CTA counts for more than a staged box or a longer list. With the list sized first, to a third of an SM, and the box
+// beside it, 31 x 31 x 9, 17 x 17 x 33, 23 x 23 x 17, 25 x 25 x 17, 41 x 41 x 5 and 13 x 13 x 65 boxes ran one or two CTAs
+// fewer (4,624, 4,194, 4,447, 3,764, 4,759 and 3,641 boxes: 731, 646, 678, 1,159, 868 and 738 us; 483, 504, 528, 418, 598
+// and 441 us so), and boxes whose tables alone exceed a third kept 2,048 voxels whatever was free (55 x 55 x 33, 400 boxes,
+// 946 -> 717 us; 73 x 73 x 9, 834 boxes, 1,565 -> 898 us; 73 x 73 x 1, 7,506 boxes, 8.86 -> 3.83 ms). A longer least list
+// costs CTAs in turn: 8,192 voxels for the larger boxes, 1,003 boxes of 41 x 41 x 65: 2.15 ms, 1.34 so.
+int pass2_plan(int max_bx, int max_dz, int K, bool* staged, Fit* fit) {
     const size_t P = (size_t)max_bx * max_bx;
     const size_t V = P * max_dz;
-    size_t budget = kStageBudget;
-    if (Pass2Layout(max_bx, max_dz, K, 0, 0, false).bytes > budget) {
-        int dev = 0, optin = 0;
-        cudaFuncAttributes fa, fq;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-            cudaFuncGetAttributes(&fa, k_pass2<256, false>) != cudaSuccess ||
-            cudaFuncGetAttributes(&fq, k_pass2_q<256, false>) != cudaSuccess)
-            return cuda_check(who);
-        const size_t st = fa.sharedSizeBytes > fq.sharedSizeBytes ? fa.sharedSizeBytes : fq.sharedSizeBytes;
-        budget = (size_t)optin > st ? (size_t)optin - st : 0;
-        if (Pass2Layout(max_bx, max_dz, K, 0, 0, false).bytes > budget)
-            return fail(XI_E_LIMIT, "pass 2: box too large (per-pixel tables exceed shared memory)");
-    }
-    // what the tables leave goes to the pixel list, then to the voxel list (beyond the room that it shares with the
-    // rocking-curve terms and the profile)
-    fit->pix = P < (size_t)kFitPix ? (int)P : kFitPix;
-    fit->cap = 0;
-    while (fit->pix > 0 && Pass2Layout(max_bx, max_dz, K, 0, fit->pix, false).bytes > budget) fit->pix /= 2;
-    const bool large = V > (size_t)XI_PASS2_LARGE_VOXELS || max_dz > XI_PASS2_LARGE_DEPTH;
-    size_t want = (size_t)g_list_cap[large ? 1 : 0];
-    const Pass2Layout base(max_bx, max_dz, K, 0, fit->pix, false);
-    auto most = [&](size_t room) {                        // voxels of a list when a CTA may use `room` bytes
-        return room > base.bytes ? ((base.pix - base.list) + (room - base.bytes)) / 16 * 16 / 8 : (size_t)0;
+    auto bytes = [&](size_t cap, size_t pix, bool box) {
+        return Pass2Layout(max_bx, max_dz, K, (int)cap, (int)pix, box).bytes;
     };
-    // the wide CTAs run three to an SM whatever their list: it takes what their share leaves
-    if (P > 200 && g_wide_nt == 256 && want) want = want > most(kPass2Share) ? want : most(kPass2Share);
-    const size_t capz = V < want ? V : want;
-    const size_t fits = most(budget);
-    fit->cap = (int)(capz < fits ? capz : fits);
-    *staged = V * sizeof(float) <= g_stage_max[1] &&
-              Pass2Layout(max_bx, max_dz, K, fit->cap, fit->pix, true).bytes <= budget;
+    const int nt = pass_threads(max_bx);
+    if (bytes(0, 0, false) > pass2_share(1, nt))
+        return fail(XI_E_LIMIT, "pass 2: box too large (per-pixel tables exceed shared memory)");
+    const bool large = V > (size_t)XI_PASS2_LARGE_VOXELS || max_dz > XI_PASS2_LARGE_DEPTH;
+    const size_t want = (size_t)g_list_cap[large ? 1 : 0], least = V < want ? V : want;
+    size_t pix = P < (size_t)kFitPix ? P : (size_t)kFitPix;
+    auto ctas = [&](bool box) {                           // an SM holds with the least list (0: not even one)
+        int n = 768 / nt;
+        while (n > 0 && bytes(least, pix, box) > pass2_share(n, nt)) --n;
+        return n;
+    };
+    const int n = ctas(false);
+    *staged = V * sizeof(float) <= g_stage_max[1] && n > 0 && ctas(true) == n;
+    const size_t room = pass2_share(n > 0 ? n : 1, nt);
+    while (pix > 0 && bytes(0, pix, *staged) > room) pix /= 2;
+    if (bytes(least, P, *staged) <= room) pix = P;
+    // voxels of a list in `room` (beyond the room that it shares with the rocking-curve terms and the profile)
+    const Pass2Layout base(max_bx, max_dz, K, 0, (int)pix, *staged);
+    const size_t most = ((base.pix - base.list) + (room - base.bytes)) / 16 * 16 / 8;
+    fit->pix = (int)pix;
+    fit->cap = want ? (int)(V < most ? V : most) : 0;
     return XI_OK;
 }
 
@@ -2120,7 +2122,7 @@ int xi_pass2(const XiDetector* det, const XiRows* R, const XiBlock* B, const flo
     const size_t P = (size_t)R->max_bx * R->max_bx;
     bool staged = false;
     Fit fit{0, 0};
-    rc = pass2_plan(R->max_bx, R->max_dz, R->K, "xi_pass2", &staged, &fit);
+    rc = pass2_plan(R->max_bx, R->max_dz, R->K, &staged, &fit);
     if (rc) return rc;
     if (staged) {
         if (P <= 96) return launch_pass2<64, true>(det, R, B, arena, prof, in, O, s, nblk, fit);
@@ -2165,7 +2167,7 @@ int xi_pass2_batched(const XiRowSet* sets, const int64_t* items, int n_items, in
     const size_t P = (size_t)max_bx * max_bx;
     bool staged = false;
     Fit fit{0, 0};
-    rc = pass2_plan(max_bx, max_dz, max_k, "xi_pass2_batched", &staged, &fit);
+    rc = pass2_plan(max_bx, max_dz, max_k, &staged, &fit);
     if (rc) return rc;
     if (staged) {
         if (P <= 96) return launch_pass2_q<64, true>(sets, items, n_items, max_bx, max_dz, max_k, fit, queue, s);
