@@ -1076,29 +1076,35 @@ constexpr int kFitWarp = 128;       // listed voxels that a warp of the fit take
 
 __host__ __device__ inline int fit_chunks(int Dz) { return (Dz + kFitChunk - 1) / kFitChunk; }
 
+// The fit's lists in shared memory: voxels, pixels listed, run bits. The bits cover the runs of every pixel where there
+// is room, so that voxels are listed also in a row with more candidate pixels than their list holds (a wide spot in a
+// 97 px box), and later rounds take only the runs that hold fitted voxels beside the list: 4,251 boxes of 97 x 97 x 1
+// 10.1 -> 6.3 ms, 160 of 97 x 97 x 65 6.2 -> 3.5 ms.
+struct Fit {
+    int cap, pix, runs;
+};
+
 // Dynamic shared memory of pass 2 for boxes up to max_bx pixels a side and max_dz bins with K neighbour columns: the
 // neighbours' frame masks (8P; first the partner's eps1 / eps2) | P2s (4P) | P2ps (4P) | background template (4P; first
 // the partner's J) | frame 64's neighbour bits (one per pixel, only when boxes reach it) | the fit list (8 x cap; first
-// the rocking-curve terms and the region's profile) | the pixels that may hold fitted voxels (2 x fitpix) | a bit for each of their
-// runs of frames | the neighbours' axis terms | staged
-// shoebox.
+// the rocking-curve terms and the region's profile) | the pixels that may hold fitted voxels (2 x fitpix) | a bit for
+// each run of frames (`runs`: of the listed pixels, or of every pixel) | the neighbours' axis terms | staged shoebox.
 struct Pass2Layout {
-    int Pm, fitpix;
+    int Pm;
     size_t p2, pp2, bref, hi, list, prof, pix, rest, nbt, stage, bytes;
 
-    __host__ __device__ Pass2Layout(int max_bx, int max_dz, int K, int cap, int fitpix_, bool staged) {
+    __host__ __device__ Pass2Layout(int max_bx, int max_dz, int K, Fit fit, bool staged) {
         Pm = max_bx * max_bx;
-        fitpix = fitpix_;
         p2 = (size_t)8 * Pm;
         pp2 = p2 + (size_t)4 * Pm;
         bref = pp2 + (size_t)4 * Pm;
         hi = bref + (size_t)4 * Pm;
         list = (hi + (max_dz > 64 ? (size_t)(Pm + 31) / 32 * 4 : 0) + 15) / 16 * 16;
         prof = list + ((size_t)max_dz * XI_RC_K * sizeof(float) + 15) / 16 * 16;
-        const size_t c = (size_t)8 * cap, t = prof - list + XI_GRID * XI_GRID * sizeof(float);
+        const size_t c = (size_t)8 * fit.cap, t = prof - list + XI_GRID * XI_GRID * sizeof(float);
         pix = list + ((c > t ? c : t) + 15) / 16 * 16;
-        rest = (pix + (size_t)2 * fitpix + 3) / 4 * 4;
-        nbt = (rest + ((size_t)fitpix * fit_chunks(max_dz) + 31) / 32 * 4 + 15) / 16 * 16;
+        rest = (pix + (size_t)2 * fit.pix + 3) / 4 * 4;
+        nbt = (rest + ((size_t)fit.runs + 31) / 32 * 4 + 15) / 16 * 16;
         stage = nbt + nb_bytes(K, max_bx, max_dz);
         bytes = stage + (staged ? ((size_t)Pm * max_dz * sizeof(float) + 15) / 16 * 16 : 0);
     }
@@ -1145,8 +1151,7 @@ template <int NT, bool STAGED>
 __device__ __forceinline__ void pass2_row(const XiDetector& det_g, const XiRows& R, const XiBlock& B,
                                           const float* __restrict__ arena, const float* __restrict__ prof,
                                           const XiPass2In& I2, const XiPass2Out& O, int row, int max_bx, int max_dz,
-                                          int cap, int fitpix, int* status, unsigned long long* bar,
-                                          unsigned& phase) {
+                                          const Fit& fit, int* status, unsigned long long* bar, unsigned& phase) {
     extern __shared__ __align__(16) unsigned char dyn2[];
     constexpr int kW = NT / 32;
     __shared__ CtaTables T;
@@ -1180,7 +1185,8 @@ __device__ __forceinline__ void pass2_row(const XiDetector& det_g, const XiRows&
         return;
     }
     const int P = bx * bx;
-    const Pass2Layout L(max_bx, max_dz, R.K, cap, fitpix, STAGED);
+    const Pass2Layout L(max_bx, max_dz, R.K, fit, STAGED);
+    const int cap = fit.cap;
     unsigned long long* nblo = reinterpret_cast<unsigned long long*>(dyn2);
     float* e1s = reinterpret_cast<float*>(dyn2);          // partner geometry, before nblo is written
     float* e2s = e1s + L.Pm;
@@ -1281,7 +1287,7 @@ __device__ __forceinline__ void pass2_row(const XiDetector& det_g, const XiRows&
     }
     if (nbhi)
         for (int w = threadIdx.x; w < (P + 31) / 32; w += NT) nbhi[w] = 0u;
-    for (int w = threadIdx.x; w < (min(P, fitpix) * fit_chunks(Dz) + 31) / 32; w += NT) rest[w] = 0u;
+    for (int w = threadIdx.x; w < (min(P * fit_chunks(Dz), fit.runs) + 31) / 32; w += NT) rest[w] = 0u;
     __syncthreads();                                      // (partner scratch free)
     float pmax = 0.0f, ppmax = 0.0f;
 #pragma unroll
@@ -1357,7 +1363,7 @@ __device__ __forceinline__ void pass2_row(const XiDetector& det_g, const XiRows&
                 int base = 0;
                 if (lane == 0) base = atomicAdd(&s_npix, __popc(ball));
                 base = __shfl_sync(0xffffffffu, base, 0) + __popc(ball & ((1u << lane) - 1u));
-                if (may && base < fitpix) pixl[base] = (unsigned short)p;
+                if (may && base < fit.pix) pixl[base] = (unsigned short)p;
             }
         }
     }
@@ -1365,10 +1371,11 @@ __device__ __forceinline__ void pass2_row(const XiDetector& det_g, const XiRows&
     // a plain row (no partner, no background template) keeps the fitted voxels' profile values, others their places
     const bool plain = !has_p && !templ;
     // ---- the fitted voxels: runs of frames of the listed pixels (of every pixel when the list overflows)
-    const bool pix_listed = s_npix <= fitpix;
+    const bool pix_listed = s_npix <= fit.pix;
     const int npix = pix_listed ? s_npix : P;
     const int nchunk = fit_chunks(Dz), clen = (Dz + nchunk - 1) / nchunk;
     const int n_run = npix * nchunk;
+    const bool kept = n_run <= fit.runs;                  // the runs have their bits (else no voxel is listed)
     // run k: its pixel and first frame; f(frame of the run, raw value, pv, ppv) for every fitted voxel of it
     auto run_of = [&](int k, int& p, int& z0) {
         const int c = k / npix, q = k - c * npix;
@@ -1426,7 +1433,7 @@ __device__ __forceinline__ void pass2_row(const XiDetector& det_g, const XiRows&
         const bool fits = at + c <= cap;
         if (c && !fits) {
             if (at < cap) s_end = at;
-            if (pix_listed) atomicOr(&rest[k >> 5], 1u << (k & 31));
+            if (kept) atomicOr(&rest[k >> 5], 1u << (k & 31));
         }
 #pragma unroll 1
         for (unsigned r = m; r; r &= r - 1u, ++at) {
@@ -1438,7 +1445,7 @@ __device__ __forceinline__ void pass2_row(const XiDetector& det_g, const XiRows&
             a8[1] += (double)(pv + ppv);
             a8[5] += (double)((pv * pv) * iv0);
             a8[6] += (double)((pv * bref) * iv0);
-            if (fits && pix_listed) {
+            if (fits && kept) {
                 ul_v[at] = net;
                 ul_i[at] = plain ? __float_as_uint(pv) : ((unsigned)z << 16) | (unsigned)p;
             }
@@ -1450,9 +1457,9 @@ __device__ __forceinline__ void pass2_row(const XiDetector& det_g, const XiRows&
     const double a110 = fmax(tot[5], 1e-12), C0 = tot[6];
     const float nuse = (float)tot[7];
     float I = (float)tot[0] / fmaxf((float)tot[1], 1e-6f), Ip = I * hp;
-    // listed voxels, and whether runs are left beside them (all of them when even the pixels overflowed their list)
-    const bool whole = pix_listed && s_nlist <= cap;
-    const int nlist = whole ? s_nlist : pix_listed ? s_end : 0;
+    // listed voxels, and whether runs are left beside them (all of them when there was no room for the runs' bits)
+    const bool whole = kept && s_nlist <= cap;
+    const int nlist = whole ? s_nlist : kept ? s_end : 0;
 
     // ---- the fit, in the first nw warps: kFitWarp listed voxels a warp, all warps when runs are left
     const int nw = whole ? min(kW, max(1, (nlist + kFitWarp - 1) / kFitWarp)) : kW;
@@ -1476,7 +1483,7 @@ __device__ __forceinline__ void pass2_row(const XiDetector& det_g, const XiRows&
         if (whole) return;
 #pragma unroll 1
         for (int k = threadIdx.x; k < n_run; k += NT) {
-            if (pix_listed && !((rest[k >> 5] >> (k & 31)) & 1u)) continue;
+            if (kept && !((rest[k >> 5] >> (k & 31)) & 1u)) continue;
             int p, z0;
             run_of(k, p, z0);
             const float bref = templ ? brefs[p] : 1.0f;
@@ -1572,8 +1579,7 @@ __global__ void __launch_bounds__(NT, min_ctas<NT>()) k_pass2(XiDetector det_g, 
                                                               const float* __restrict__ arena,
                                                               const float* __restrict__ prof, XiPass2In I2,
                                                               XiPass2Out O, const int32_t* __restrict__ order,
-                                                              int max_bx, int max_dz, int cap, int fitpix,
-                                                              int* status) {
+                                                              int max_bx, int max_dz, Fit fit, int* status) {
     __shared__ __align__(8) unsigned long long s_bar;
     if (STAGED) {
         if (threadIdx.x == 0) mbar_init(&s_bar, 1);
@@ -1581,15 +1587,15 @@ __global__ void __launch_bounds__(NT, min_ctas<NT>()) k_pass2(XiDetector det_g, 
     }
     unsigned phase = 0;
     pass2_row<NT, STAGED>(det_g, R, B, arena, prof, I2, O, order ? order[blockIdx.x] : blockIdx.x, max_bx, max_dz,
-                          cap, fitpix, status, &s_bar, phase);
+                          fit, status, &s_bar, phase);
 }
 
 // Pass 2 over a queue of (set, row) items (as k_pass1_q); a set's pass-1 outputs are its pass-2 inputs.
 template <int NT, bool STAGED>
 __global__ void __launch_bounds__(NT, min_ctas<NT>()) k_pass2_q(const XiRowSet* __restrict__ sets,
                                                                 const int64_t* __restrict__ items, int n_items,
-                                                                int max_bx, int max_dz, int max_k, int cap,
-                                                                int fitpix, int* queue, int* status) {
+                                                                int max_bx, int max_dz, int max_k, Fit fit,
+                                                                int* queue, int* status) {
     __shared__ __align__(8) unsigned long long s_bar;
     __shared__ XiRowSet s_set;
     __shared__ int s_item, s_cur;
@@ -1620,7 +1626,7 @@ __global__ void __launch_bounds__(NT, min_ctas<NT>()) k_pass2_q(const XiRowSet* 
         in.bg = s_set.p1.bg;
         in.nbg = s_set.p1.nbg;
         pass2_row<NT, STAGED>(s_set.det, s_set.rows, s_set.blk, s_set.arena, s_set.prof, in, s_set.p2,
-                              (int)(v & 0xffffffffll), max_bx, max_dz, cap, fitpix, status, &s_bar, phase);
+                              (int)(v & 0xffffffffll), max_bx, max_dz, fit, status, &s_bar, phase);
     }
 }
 
@@ -1902,20 +1908,15 @@ int launch_pass1(const XiDetector* det, const XiRows* R, const XiBlock* B, const
     return cuda_check("xi_pass1");
 }
 
-// The fit's shared-memory plan of a launch: voxels of the fit list, pixels listed for it.
-struct Fit {
-    int cap, pix;
-};
-
 template <int NT, bool STAGED>
 int launch_pass2(const XiDetector* det, const XiRows* R, const XiBlock* B, const float* arena, const float* prof,
                  const XiPass2In* in, XiPass2Out* O, cudaStream_t s, int nblk, Fit fit) {
-    const size_t sm = Pass2Layout(R->max_bx, R->max_dz, R->K, fit.cap, fit.pix, STAGED).bytes;
+    const size_t sm = Pass2Layout(R->max_bx, R->max_dz, R->K, fit, STAGED).bytes;
     cudaFuncSetAttribute(k_pass2<NT, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     cudaFuncSetAttribute(k_pass2<NT, STAGED>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          cudaSharedmemCarveoutMaxShared);
     k_pass2<NT, STAGED><<<nblk, NT, sm, s>>>(*det, *R, *B, arena, prof, *in, *O, R->order, R->max_bx, R->max_dz,
-                                              fit.cap, fit.pix, status_ptr());
+                                              fit, status_ptr());
     return cuda_check("xi_pass2");
 }
 
@@ -1950,15 +1951,14 @@ int launch_pass1_q(const XiRowSet* sets, const int64_t* items, int n_items, int 
 template <int NT, bool STAGED>
 int launch_pass2_q(const XiRowSet* sets, const int64_t* items, int n_items, int max_bx, int max_dz, int K, Fit fit,
                    int* queue, cudaStream_t s) {
-    const size_t sm = Pass2Layout(max_bx, max_dz, K, fit.cap, fit.pix, STAGED).bytes;
+    const size_t sm = Pass2Layout(max_bx, max_dz, K, fit, STAGED).bytes;
     cudaFuncSetAttribute(k_pass2_q<NT, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     cudaFuncSetAttribute(k_pass2_q<NT, STAGED>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          cudaSharedmemCarveoutMaxShared);
     const int grid = resident_grid(k_pass2_q<NT, STAGED>, NT, sm, n_items);
     if (grid <= 0) return cuda_check("xi_pass2_batched: occupancy");
     k_zero_int<<<1, 1, 0, s>>>(queue);
-    k_pass2_q<NT, STAGED><<<grid, NT, sm, s>>>(sets, items, n_items, max_bx, max_dz, K, fit.cap, fit.pix, queue,
-                                                   status_ptr());
+    k_pass2_q<NT, STAGED><<<grid, NT, sm, s>>>(sets, items, n_items, max_bx, max_dz, K, fit, queue, status_ptr());
     return cuda_check("xi_pass2_batched");
 }
 
@@ -1992,8 +1992,8 @@ int pass_threads(int max_bx) {
 // Pass 2's shared-memory plan for boxes up to max_bx pixels a side and max_dz bins with K neighbour columns: whether
 // the box is staged, and the fit's lists. First the CTAs that an SM holds: as many as the registers allow, fewer where
 // the tables with the least list (g_list_cap voxels, or the whole box) need more room than their share. Then what that
-// share leaves goes to the box, staged where it is small and costs no CTA, to the list of pixels (all of the box's where
-// the least list still fits, else kFitPix) and to the list of voxels. Runs that
+// share leaves goes to the box, staged where it is small and costs no CTA, to the runs' bits and the list of pixels (of all of
+// the box's pixels where the least list still fits, else of kFitPix) and to the list of voxels. Runs that
 // do not fit the list are taken from the box in every round; the second least list is for launches whose largest box
 // exceeds XI_PASS2_LARGE_VOXELS voxels or XI_PASS2_LARGE_DEPTH bins; 0 voxels: no list.
 // A CTA counts for more than a staged box or a longer list. With the list sized first, to a third of an SM, and the box
@@ -2005,30 +2005,35 @@ int pass_threads(int max_bx) {
 int pass2_plan(int max_bx, int max_dz, int K, bool* staged, Fit* fit) {
     const size_t P = (size_t)max_bx * max_bx;
     const size_t V = P * max_dz;
-    auto bytes = [&](size_t cap, size_t pix, bool box) {
-        return Pass2Layout(max_bx, max_dz, K, (int)cap, (int)pix, box).bytes;
+    const size_t chunks = (size_t)fit_chunks(max_dz);
+    auto lists = [&](size_t cap, size_t pix, size_t run_pix) {
+        return Fit{(int)cap, (int)pix, (int)(run_pix * chunks)};
+    };
+    auto bytes = [&](size_t cap, size_t pix, size_t run_pix, bool box) {
+        return Pass2Layout(max_bx, max_dz, K, lists(cap, pix, run_pix), box).bytes;
     };
     const int nt = pass_threads(max_bx);
-    if (bytes(0, 0, false) > pass2_share(1, nt))
+    if (bytes(0, 0, 0, false) > pass2_share(1, nt))
         return fail(XI_E_LIMIT, "pass 2: box too large (per-pixel tables exceed shared memory)");
     const bool large = V > (size_t)XI_PASS2_LARGE_VOXELS || max_dz > XI_PASS2_LARGE_DEPTH;
     const size_t want = (size_t)g_list_cap[large ? 1 : 0], least = V < want ? V : want;
     size_t pix = P < (size_t)kFitPix ? P : (size_t)kFitPix;
     auto ctas = [&](bool box) {                           // an SM holds with the least list (0: not even one)
         int n = 768 / nt;
-        while (n > 0 && bytes(least, pix, box) > pass2_share(n, nt)) --n;
+        while (n > 0 && bytes(least, pix, pix, box) > pass2_share(n, nt)) --n;
         return n;
     };
     const int n = ctas(false);
     *staged = V * sizeof(float) <= g_stage_max[1] && n > 0 && ctas(true) == n;
     const size_t room = pass2_share(n > 0 ? n : 1, nt);
-    while (pix > 0 && bytes(0, pix, *staged) > room) pix /= 2;
-    if (bytes(least, P, *staged) <= room) pix = P;
+    while (pix > 0 && bytes(0, pix, pix, *staged) > room) pix /= 2;
+    size_t run_pix = pix;
+    if (bytes(least, pix, P, *staged) <= room) run_pix = P;
+    if (bytes(least, P, P, *staged) <= room) pix = P;
     // voxels of a list in `room` (beyond the room that it shares with the rocking-curve terms and the profile)
-    const Pass2Layout base(max_bx, max_dz, K, 0, (int)pix, *staged);
+    const Pass2Layout base(max_bx, max_dz, K, lists(0, pix, run_pix), *staged);
     const size_t most = ((base.pix - base.list) + (room - base.bytes)) / 16 * 16 / 8;
-    fit->pix = (int)pix;
-    fit->cap = want ? (int)(V < most ? V : most) : 0;
+    *fit = lists(want ? (V < most ? V : most) : 0, pix, run_pix);
     return XI_OK;
 }
 
@@ -2121,7 +2126,7 @@ int xi_pass2(const XiDetector* det, const XiRows* R, const XiBlock* B, const flo
     cudaStream_t s = (cudaStream_t)stream;
     const size_t P = (size_t)R->max_bx * R->max_bx;
     bool staged = false;
-    Fit fit{0, 0};
+    Fit fit{0, 0, 0};
     rc = pass2_plan(R->max_bx, R->max_dz, R->K, &staged, &fit);
     if (rc) return rc;
     if (staged) {
@@ -2166,7 +2171,7 @@ int xi_pass2_batched(const XiRowSet* sets, const int64_t* items, int n_items, in
     cudaStream_t s = (cudaStream_t)stream;
     const size_t P = (size_t)max_bx * max_bx;
     bool staged = false;
-    Fit fit{0, 0};
+    Fit fit{0, 0, 0};
     rc = pass2_plan(max_bx, max_dz, max_k, &staged, &fit);
     if (rc) return rc;
     if (staged) {
