@@ -9,11 +9,13 @@
 // sums of value and square are one packed float pair (add.rn.f32x2: two IEEE adds an instruction); the counts are
 // integers (bit windows along x, running sums along y); the tests' roots and quotients are computed only where bounds
 // leave the test open. One warp a CTA: with four, and a strip of 256 columns, warps waited for one another (1.6 ms in
-// place of 1.4 at that stage). Against one thread a pixel with both window loops in shared memory (32 x 8 tiles, 46 x
-// 22 staged for the second pass): four 4148 x 4362 frames 4.19 -> 1.13 ms, one 1030 x 1065 frame 88 -> 50 us
-// (first pass alone: 1.35 -> 0.38 ms, 38 -> 34 us).
+// place of 1.4 at that stage). Against a thread a pixel with both window loops in shared memory (32 x 8 tiles, 46 x
+// 22 staged for the second pass): four 4148 x 4362 frames 4.19 -> 1.13 ms, one 1030 x 1065 frame 76 -> 44 us
+// (first pass alone: 1.35 -> 0.38 ms, 26 -> 18 us), windows of half widths 0 to 8, square and not, of four such frames
+// 0.27 to 0.56 of the time.
 // The first launch of an extended call finds the strong pixels and writes the background pixels (those not within
 // 1 px of one) and the pixels within 2 px of one; the second re-estimates the background and classifies.
+// Small frames have too few strips for that (a warp's march is one long chain of steps); they take the tiles (below).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -48,8 +50,8 @@ __device__ __forceinline__ void unpack2(pair_t v, float& a, float& b) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
 
-// Shared memory of a CTA for half widths hx, hy: the ring of horizontal sums (2 hy + 4 rows) and counts, two buffers
-// of four staged rows of values and of weight bits, the bit rows of the first pass.
+// Shared memory of a CTA for half widths hx, hy: the ring of horizontal sums (2 hy + 4 rows) and counts, four staged
+// rows of values and of weight bits, the bit rows of the first pass (25.6 KB at most).
 struct Layout {
     int ring, width, words;                  // rows of the ring; staged values and weight words of a row
     size_t cnt, raw, bits, flag, bytes;
@@ -66,7 +68,7 @@ struct Layout {
     }
 };
 
-// The window sums of the CTA's strip: columns x0 .. x0 + 255, four rows a step, a thread's two columns in its
+// The window sums of the CTA's strip: columns x0 .. x0 + 63, four rows a step, a thread's two columns in its
 // registers. H >= 0: both half widths, known at compile time (loops unrolled); H < 0: hx, hy. A pixel enters with
 // weight 1 where it is valid (SEL false) or where its flag in sel is set.
 template <int H, bool SEL>
@@ -410,20 +412,161 @@ __global__ void __launch_bounds__(kNT) k_spot_extended(const float* __restrict__
     }
 }
 
+// ---- tiles: a thread a pixel, a CTA a 32 x 8 tile of one frame. The tile and its halo are staged in shared memory, summed
+// along x for every staged row, then along y for every pixel, in the same order as the strips' sums.
+
+constexpr int kTW = 32, kTH = 8, kTile = kTW * kTH;
+
+// window sums of the valid-pixel count, the values and their squares
+struct Sums {
+    float n, s1, s2;
+};
+
+// The sums of this thread's pixel over the pixels that enter: the valid ones, or those whose flag in sel is set.
+__device__ Sums tile_sums(const float* __restrict__ img, const uint8_t* __restrict__ sel, int ny, int nx, int hx, int hy,
+                          float* sm) {
+    const int W = kTW + 2 * hx, H = kTH + 2 * hy;
+    float* tw = sm;                   // staged weights, H x W
+    float* tx = tw + H * W;           // staged values
+    float* hw = tx + H * W;           // sums along x, H x kTW
+    float* hs = hw + H * kTW;
+    float* hq = hs + H * kTW;
+    const int x0 = blockIdx.x * kTW - hx, y0 = blockIdx.y * kTH - hy;
+    for (int i = threadIdx.x; i < H * W; i += kTile) {
+        const int r = i / W, c = i % W;
+        const int y = y0 + r, x = x0 + c;
+        float w = 0.0f, v = 0.0f;
+        if (y >= 0 && y < ny && x >= 0 && x < nx) {
+            const size_t k = (size_t)y * nx + x;
+            const float p = img[k];
+            const bool on = sel ? sel[k] != 0 : p >= 0.0f;
+            w = on ? 1.0f : 0.0f;
+            v = on ? p : 0.0f;
+        }
+        tw[i] = w;
+        tx[i] = v;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < H * kTW; i += kTile) {
+        const int r = i / kTW, c = i % kTW;
+        float a = 0.0f, s = 0.0f, q = 0.0f;
+        for (int d = 0; d <= 2 * hx; ++d) {
+            const float v = tx[r * W + c + d];
+            a = a + tw[r * W + c + d];
+            s = s + v;
+            q = q + v * v;
+        }
+        hw[i] = a;
+        hs[i] = s;
+        hq[i] = q;
+    }
+    __syncthreads();
+    const int r = threadIdx.x / kTW, c = threadIdx.x % kTW;
+    Sums o{0.0f, 0.0f, 0.0f};
+    for (int d = 0; d <= 2 * hy; ++d) {
+        const int k = (r + d) * kTW + c;
+        o.n = o.n + hw[k];
+        o.s1 = o.s1 + hs[k];
+        o.s2 = o.s2 + hq[k];
+    }
+    return o;
+}
+
+size_t tile_smem(int hx, int hy) {                         // (38.3 KB at most)
+    const size_t W = kTW + 2 * hx, H = kTH + 2 * hy;
+    return (2 * H * W + 3 * H * kTW) * sizeof(float);
+}
+
+__device__ bool any_flag(const uint8_t* f, int ny, int nx, int y, int x, int r) {
+    for (int yy = max(y - r, 0); yy <= min(y + r, ny - 1); ++yy)
+        for (int xx = max(x - r, 0); xx <= min(x + r, nx - 1); ++xx)
+            if (f[(size_t)yy * nx + xx]) return true;
+    return false;
+}
+
+// the dispersion test: first-pass strong mask and local mean
+__global__ void __launch_bounds__(kTile) k_spot_tile_first(const float* __restrict__ img, int ny, int nx, int hx, int hy,
+                                                           float gain, float n_s, float min_local,
+                                                           uint8_t* __restrict__ strong, float* __restrict__ mean) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    const size_t f0 = (size_t)blockIdx.z * ny * nx;
+    const Sums t = tile_sums(img + f0, nullptr, ny, nx, hx, hy, reinterpret_cast<float*>(sm));
+    const int y = blockIdx.y * kTH + threadIdx.x / kTW, x = blockIdx.x * kTW + threadIdx.x % kTW;
+    if (y >= ny || x >= nx) return;
+    const size_t k = f0 + (size_t)y * nx + x;
+    const float p = img[k];
+    strong[k] = p >= 0.0f && t.n >= min_local && dispersed(p, t.n, t.s1, t.s2, gain, n_s) ? 1 : 0;
+    mean[k] = t.s1 / fmaxf(t.n, 2.0f);
+}
+
+// the background pixels of the extended pass
+__global__ void __launch_bounds__(kTile) k_spot_tile_background(const float* __restrict__ img, int ny, int nx,
+                                                                const uint8_t* __restrict__ strong,
+                                                                const float* __restrict__ mean, float gain, float bgp,
+                                                                uint8_t* __restrict__ bg) {
+    const int y = blockIdx.y * kTH + threadIdx.x / kTW, x = blockIdx.x * kTW + threadIdx.x % kTW;
+    if (y >= ny || x >= nx) return;
+    const size_t f0 = (size_t)blockIdx.z * ny * nx, k = f0 + (size_t)y * nx + x;
+    const float p = img[k], m = mean[k];
+    const float sigma = sqrtf(gain * fmaxf(m, 0.5f));
+    bg[k] = p >= 0.0f && !any_flag(strong + f0, ny, nx, y, x, 1) && p <= m + bgp * sigma ? 1 : 0;
+}
+
+// the extended pass
+__global__ void __launch_bounds__(kTile) k_spot_tile_extended(const float* __restrict__ img, int ny, int nx, int hx,
+                                                              int hy, float gain, float sp, float min_local4,
+                                                              const uint8_t* __restrict__ bg,
+                                                              const uint8_t* __restrict__ first,
+                                                              uint8_t* __restrict__ strong, float* __restrict__ mean) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    const size_t f0 = (size_t)blockIdx.z * ny * nx;
+    const Sums t = tile_sums(img + f0, bg + f0, ny, nx, hx, hy, reinterpret_cast<float*>(sm));
+    const int y = blockIdx.y * kTH + threadIdx.x / kTW, x = blockIdx.x * kTW + threadIdx.x % kTW;
+    if (y >= ny || x >= nx) return;
+    const size_t k = f0 + (size_t)y * nx + x;
+    const float p = img[k];
+    const bool st = p >= 0.0f && t.n >= min_local4 && exceeds(p, t.n, t.s1, t.s2, gain, sp);
+    strong[k] = st && any_flag(first + f0, ny, nx, y, x, 2) ? 1 : 0;
+    mean[k] = t.s1 / fmaxf(t.n, 2.0f);
+}
+
+// ---- the choice
+
+constexpr int kSms = 148;                    // of a B200
+
+// CTAs of strips of `rows` rows
+int64_t strip_ctas(bool extended, int n_frames, int ny, int nx, int rows) {
+    const int cols = extended ? kCols - 4 : kCols;
+    return (int64_t)((nx + cols - 1) / cols) * ((ny + rows - 1) / rows) * n_frames;
+}
+
+// Strips where they are enough to hide a march's latency, else tiles. Strips of few rows recompute the rows of their
+// windows above them: square windows with unrolled loops (half widths 2 to 4) still gain in four rows, the others
+// want strips of twelve, the widest extended ones more of them. One frame, strips against tiles:
+//   half width 3: 260 x 256 7.7 / 8.0 us plain, 23 / 19 extended; 512 x 512 9 / 11, 26 / 29; 768 x 768 11 / 16, 35 / 50
+//   half width 5: 512 x 512 12.8 / 12.2 plain, 43 / 35 extended; 768 x 768 16 / 20, 81 / 64; 1000 x 1000 26 / 31, 73 / 97
+//   half width 8: 260 x 256 17 / 9, 60 / 24; 896 x 900 34 / 33, 163 / 117; 1030 x 1065 32 / 42, 139 / 146
+constexpr int kWideCtas = kSms * 12;
+bool use_strips(const XiSpotParams& p, int n_frames, int ny, int nx) {
+    const bool ext = p.extended != 0;
+    const int wide = p.nbx > p.nby ? p.nbx : p.nby;
+    if (p.nbx == p.nby && wide >= 2 && wide <= 4) return strip_ctas(ext, n_frames, ny, nx, 4) >= kSms * (ext ? 6 : 3);
+    if (!ext && wide < 7) return strip_ctas(ext, n_frames, ny, nx, 4) >= kSms * 10;
+    return strip_ctas(ext, n_frames, ny, nx, 12) >= (ext && wide >= 7 ? kWideCtas : kSms * 8);
+}
+
 // Rows a CTA marches down: long strips recompute little (the 2 hy rows above the first one), short ones fill the
-// device: the longest of 60, 28 and 12 that gives every SM eight CTAs, else 4. (Four fewer than a multiple of the step:
-// an extended first pass computes two rows more above and below.) A 1030 x 1065 frame takes 12 (50 us; 66 with 4, the
-// choice if sixteen CTAs an SM were asked for).
+// device: the longest of 60, 28 and 12 that gives every SM eight CTAs, else 4. (All of them 4 k: an extended first pass
+// computes two rows more above and below, which are whole steps too.)
 int strip_rows(int n_frames, int ny, int strips) {
     for (int rows : {60, 28, 12})
-        if ((int64_t)strips * ((ny + rows - 1) / rows) * n_frames >= 148 * 8) return rows;
+        if ((int64_t)strips * ((ny + rows - 1) / rows) * n_frames >= kSms * 8) return rows;
     return 4;
 }
 
 template <typename K, typename... A>
 void launch(K kernel, int cols, int hx, int hy, int n_frames, int ny, int nx, cudaStream_t s, const float* img, A... a) {
     const size_t sm = Layout(hx, hy).bytes;
-    if (sm > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     const int strips = (nx + cols - 1) / cols, rows = strip_rows(n_frames, ny, strips);
     kernel<<<dim3((unsigned)strips, (unsigned)((ny + rows - 1) / rows), (unsigned)n_frames), kNT, sm, s>>>(
         img, ny, nx, hx, hy, rows, a...);
@@ -454,7 +597,9 @@ void launch_extended(int hx, int hy, int n_frames, int ny, int nx, cudaStream_t 
 extern "C" size_t xi_spot_workspace(int n_frames, int ny, int nx) {
     if (n_frames < 0 || ny < 0 || nx < 0) return 0;
     const size_t n = (size_t)n_frames * ny * nx;
-    return ((n + 255) / 256 * 256) * 2;          // the first pass's flags: near a strong pixel, background
+    const size_t flags = (n + 255) / 256 * 256;
+    // the first pass's flags (strong, or near a strong pixel; background), and its mean where a window may take tiles
+    return 2 * flags + (strip_ctas(true, n_frames, ny, nx, 12) < kWideCtas ? n * sizeof(float) : 0);
 }
 
 extern "C" int xi_spot_strong(const float* img, int n_frames, int ny, int nx, float gain, const XiSpotParams* p,
@@ -468,6 +613,13 @@ extern "C" int xi_spot_strong(const float* img, int n_frames, int ny, int nx, fl
     if (n_frames > 65535) return xi_fail(XI_E_LIMIT, "xi_spot_strong: more than 65535 frames in one call");
     cudaStream_t s = (cudaStream_t)stream;
     const float ml = (float)p->min_local;
+    const bool strips = use_strips(*p, n_frames, ny, nx);
+    const dim3 grid((unsigned)((nx + kTW - 1) / kTW), (unsigned)((ny + kTH - 1) / kTH), (unsigned)n_frames);
+    if (!p->extended && !strips) {
+        k_spot_tile_first<<<grid, kTile, tile_smem(p->nbx, p->nby), s>>>(img, ny, nx, p->nbx, p->nby, gain,
+                                                                         p->signal_pixel, ml, strong, mean);
+        return xi_cuda_check("xi_spot_strong");
+    }
     if (!p->extended) {
         launch_first<false>(p->nbx, p->nby, kCols, n_frames, ny, nx, s, img, gain, p->signal_pixel, ml, 0.0f, strong,
                             (uint8_t*)nullptr, mean);
@@ -476,6 +628,17 @@ extern "C" int xi_spot_strong(const float* img, int n_frames, int ny, int nx, fl
     if (!ws || ws_bytes < xi_spot_workspace(n_frames, ny, nx)) return xi_fail(XI_E_ARG, "xi_spot_strong: workspace");
     uint8_t* near = static_cast<uint8_t*>(ws);
     uint8_t* bg = near + (n + 255) / 256 * 256;
+    if (!strips) {
+        uint8_t* first = near;
+        float* mean1 = reinterpret_cast<float*>(bg + (n + 255) / 256 * 256);
+        const int hx2 = 2 * p->nbx + 1, hy2 = 2 * p->nby + 1;
+        k_spot_tile_first<<<grid, kTile, tile_smem(p->nbx, p->nby), s>>>(img, ny, nx, p->nbx, p->nby, gain,
+                                                                         p->signal_pixel, ml, first, mean1);
+        k_spot_tile_background<<<grid, kTile, 0, s>>>(img, ny, nx, first, mean1, gain, p->background_pixel, bg);
+        k_spot_tile_extended<<<grid, kTile, tile_smem(hx2, hy2), s>>>(img, ny, nx, hx2, hy2, gain, p->signal_pixel,
+                                                                      4.0f * ml, bg, first, strong, mean);
+        return xi_cuda_check("xi_spot_strong");
+    }
     launch_first<true>(p->nbx, p->nby, kCols - 4, n_frames, ny, nx, s, img, gain, p->signal_pixel, ml,
                        p->background_pixel, near, bg, (float*)nullptr);
     launch_extended(2 * p->nbx + 1, 2 * p->nby + 1, n_frames, ny, nx, s, img, gain, p->signal_pixel, 4.0f * ml, bg, near,
