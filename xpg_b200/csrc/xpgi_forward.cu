@@ -212,8 +212,14 @@ int launch_check(const char* who) {
 }
 
 // A warp a reflection where that fills the device, else a CTA (the two gathers of 60,000 boxes of 9 x 13 x 13 voxels:
-// 472 and 371 us by warps, 515 and 427 by CTAs; of 5,000 boxes 57 and 52 us by warps, 52 and 45 by CTAs).
-bool warp_rows(const XiFmBoxes& B) { return B.n >= 148 * 64; }
+// 472 and 371 us by warps, 515 and 427 by CTAs; of 5,000 boxes 57 and 52 us by warps, 52 and 45 by CTAs). A box of at
+// most 32 pixels has no work for a second warp, one of up to 64 little: warps too, from 148 x 8 rows on of the latter
+// (ratio gather of 9,471 boxes of 3 x 1 x 1 with three terms 27.1 us by CTAs, 11.2 by warps, of 1 x 7 x 7 14.4 and 8.1;
+// 2,000 of 9 x 7 x 7 8.6 and 7.3, but 500 of them 5.1 and 6.1).
+bool warp_rows(const XiFmBoxes& B) {
+    const int64_t px = (int64_t)B.b * B.b;
+    return B.n >= 148 * 64 || px <= 32 || (px <= 64 && B.n >= 148 * 8);
+}
 
 template <int T>
 void launch_scatter(const XiFmBoxes& B, const XiFmWindow& W, const float* I, const float* beta, float* mu,
