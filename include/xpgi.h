@@ -126,6 +126,7 @@ typedef struct {
     const int64_t *cnt_off;         /* offset of the row's Dz bin counters in `cnt` (binned rows), else -1 */
     const int32_t *order;           /* (n_order) rows processed by the call (NULL: rows 0..n-1) */
     int n_order;
+    int max_bx;                     /* largest side of the rows, 0: not known (chooses the launch, not the results) */
 } XiGatherRows;
 
 /* Frames of a gather call. Frame w of the wedge is frame index first_fi + w (0-based). */

@@ -426,9 +426,17 @@ constexpr int kZBatch = 8;          // and pass C, whose frame sums go by eights
 // (15 of 20 stall cycles) and by how many frames' pages are open at once: more frames in flight a thread make it slower
 // (16 frames: 16.7 ms for the 16M-pixel sweep's 107,446 rows), more pixels of the same frames faster. 128 threads and
 // 8 frames: 5.94 ms there and 5.10 ms for the 4M-pixel sweep's 90,287; 256 and 4: 5.06 and 4.44 ms; 512 and 4: 4.80 and
-// 4.96 ms.
+// 4.96 ms; 128 and 4: 5.75 and 4.96 ms. Two rules beside that:
+// - where the launch's largest box is known to have no more than 128 pixels, 128 threads: the others only kept rows off
+//   the SM (30,000 boxes of 9 x 9 x 5: 70 us with 128 and 8 frames, 79 with 256 and 4, 59 with 128 and 4; a fifth of the
+//   rows, 11, 13.5 and 11). Not from 13 px on: 100 boxes of 13 x 13 x 17 6.6 us with 256, 9.4 with 128, 10,000 of
+//   17 x 17 x 33 234 and 278.
+// - float frames, which are not encoded after the load, are bound by the loads in flight: 128 threads up to 17 px (23,068
+//   boxes of 17 x 17 x 9: 134 us with 128 and 8 frames, 146 with 256 and 4, 133 so), eight frames a thread from there on
+//   (1,250 boxes of 73 x 73 x 9: 133, 149 and 132 us).
 constexpr int kGatherThreads = 256;
-constexpr int kGatherBatch = 4;
+constexpr int kGatherSmall = 11, kGatherSmallFloat = 17;  // largest side of a launch with half the threads
+constexpr int kGatherBatch = 4, kGatherFloatBatch = 8;
 
 // Dynamic shared memory of pass 1 for boxes up to max_bx pixels a side and max_dz bins with K neighbour columns: the
 // neighbours' frame masks (8P) | geometry scratch eps1, then the background template (4P) | eps2, then the img2 counts
@@ -1692,7 +1700,8 @@ __device__ __forceinline__ float box_value(const XiFrames& F, const void* frame,
     return sum;
 }
 
-// The gather of one row's box from the frames of a wedge, by the whole CTA.
+// The gather of one row's box from the frames of a wedge, by the whole CTA; plain rows NB frames at a time.
+template <int NB>
 __device__ __forceinline__ void gather_row(const XiFrames& F, const XiGatherRows& G, float* __restrict__ arena,
                                            int32_t* __restrict__ cnt, int row) {
     const int iz0 = G.iz0[row], fb = G.fb[row], Dz = G.Dz[row], bx = G.bx[row];
@@ -1704,8 +1713,8 @@ __device__ __forceinline__ void gather_row(const XiFrames& F, const XiGatherRows
     float* dst = arena + G.sb_off[row];
     const size_t fstride = (size_t)F.ny * F.nx * (F.is_float ? sizeof(float) : sizeof(uint32_t));
     if (fb == 1 && s == 1) {
-        // plain rows: a thread owns box pixels and reads a pixel's frames kGatherBatch at a time (independent loads
-        // in flight); the pixel's bounds and mask are looked up once
+        // plain rows: a thread owns box pixels and reads a pixel's frames NB at a time (independent loads in flight);
+        // the pixel's bounds and mask are looked up once
         const size_t fpix = (size_t)F.ny * F.nx;
         for (int p = threadIdx.x; p < P; p += blockDim.x) {
             const int y = iy0 + p / bx, x = ix0 + p % bx;
@@ -1713,10 +1722,10 @@ __device__ __forceinline__ void gather_row(const XiFrames& F, const XiGatherRows
             const size_t idx = inside ? (size_t)y * F.nx + x : 0;
             const bool masked = inside && F.mask && F.mask[idx] == 0;
             const int k0 = F.first_fi - iz0;                  // box frame of wedge frame 0
-            for (int w = w0; w < w1; w += kGatherBatch) {
-                float vv[kGatherBatch];
+            for (int w = w0; w < w1; w += NB) {
+                float vv[NB];
 #pragma unroll
-                for (int u = 0; u < kGatherBatch; ++u) {
+                for (int u = 0; u < NB; ++u) {
                     vv[u] = -1.0f;
                     const int ww = w + u;
                     if (inside && ww < w1) {
@@ -1725,7 +1734,7 @@ __device__ __forceinline__ void gather_row(const XiFrames& F, const XiGatherRows
                     }
                 }
 #pragma unroll
-                for (int u = 0; u < kGatherBatch; ++u) {
+                for (int u = 0; u < NB; ++u) {
                     const int ww = w + u;
                     if (ww >= w1 || (F.frame_ok && !F.frame_ok[ww])) continue;
                     const float v = masked ? fminf(vv[u], -1.0f) : vv[u];
@@ -1760,9 +1769,10 @@ __device__ __forceinline__ void gather_row(const XiFrames& F, const XiGatherRows
     }
 }
 
+template <int NB>
 __global__ void k_gather(XiFrames F, XiGatherRows G, float* __restrict__ arena, int32_t* __restrict__ cnt,
                          const int32_t* __restrict__ order) {
-    gather_row(F, G, arena, cnt, order ? order[blockIdx.x] : blockIdx.x);
+    gather_row<NB>(F, G, arena, cnt, order ? order[blockIdx.x] : blockIdx.x);
 }
 
 // The gather of one wedge with the frames and rows read from a device descriptor when the kernel runs, so that one
@@ -1772,7 +1782,7 @@ __global__ void k_gather_step(const XiGatherStep* __restrict__ step, XiGatherRow
     const XiFrames F = step->frames;
     const int n = step->n_order;
     if (F.n_frames <= 0) return;
-    for (int k = blockIdx.x; k < n; k += gridDim.x) gather_row(F, G, arena, cnt, step->order[k]);
+    for (int k = blockIdx.x; k < n; k += gridDim.x) gather_row<kGatherBatch>(F, G, arena, cnt, step->order[k]);
 }
 
 
@@ -2209,7 +2219,11 @@ int xi_gather(const XiFrames* F, const XiGatherRows* G, float* arena, int32_t* c
     if (F->n_frames < 0 || F->ny <= 0 || F->nx <= 0 || G->n < 0) return fail(XI_E_ARG, "xi_gather: bad sizes");
     const int nblk = G->order ? G->n_order : G->n;
     if (nblk == 0 || F->n_frames == 0) return XI_OK;
-    k_gather<<<nblk, kGatherThreads, 0, (cudaStream_t)stream>>>(*F, *G, arena, cnt, G->order);
+    const bool small = G->max_bx > 0 && G->max_bx <= (F->is_float ? kGatherSmallFloat : kGatherSmall);
+    const int nt = small ? kGatherThreads / 2 : kGatherThreads;
+    cudaStream_t s = (cudaStream_t)stream;
+    if (F->is_float && !small) k_gather<kGatherFloatBatch><<<nblk, nt, 0, s>>>(*F, *G, arena, cnt, G->order);
+    else k_gather<kGatherBatch><<<nblk, nt, 0, s>>>(*F, *G, arena, cnt, G->order);
     return cuda_check("xi_gather");
 }
 

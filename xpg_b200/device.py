@@ -552,6 +552,7 @@ class GatherRows:
             setattr(g, k, N.ptr(v))
         g.order = None
         g.n_order = 0
+        g.max_bx = int(rows.bx.max()) if n else 0
         self.s = g
         self.span = rows.Dz * fb
         self.binned = binned

@@ -57,7 +57,7 @@ class XiPass2Out(C.Structure):
 
 class XiGatherRows(C.Structure):
     _fields_ = [("n", C.c_int), ("ix0", _fp), ("iy0", _fp), ("iz0", _fp), ("fb", _fp), ("Dz", _fp), ("bx", _fp),
-                ("pxs", _fp), ("sb_off", _fp), ("cnt_off", _fp), ("order", _fp), ("n_order", C.c_int)]
+                ("pxs", _fp), ("sb_off", _fp), ("cnt_off", _fp), ("order", _fp), ("n_order", C.c_int), ("max_bx", C.c_int)]
 
 
 class XiFrames(C.Structure):
