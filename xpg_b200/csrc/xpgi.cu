@@ -403,8 +403,8 @@ __device__ void stage_wait(bool tma, unsigned long long* bar, unsigned parity, f
     bool ok = true;
     if (tma) ok = mbar_wait(bar, parity, 1ll << 24);
     if (!tma || !ok) {
-        if (!ok && threadIdx.x == 0) atomicOr(status, 2);
-        __syncthreads();
+        // (no barrier here: the wait may run out for some threads only; the others' share has arrived by the copy)
+        if (!ok) atomicOr(status, 2);
         for (int v = threadIdx.x; v < V; v += blockDim.x) stage[v] = sb[v];
     } else {
         // the bulk copy moved whole 16-byte units; the last 0..3 values come with plain loads (no read past the row)
