@@ -4,10 +4,12 @@ A batched launch sizes its shared memory, threads per CTA and staging for the la
 put small boxes in CTAs sized for large ones (fewer resident CTAs), narrow bins make more launches (more tails). The
 CTA shape of large boxes (128 threads at 6 CTAs per SM, or 256 at 3), the largest box staged in shared memory by
 a bulk copy, and pass 2's least fit-list capacity (the fitted voxels kept in shared memory for its six IRLS iterations;
-the rest comes from the box each time) trade resident reflections per SM against work per CTA. The tuner
-times pass 1 and pass 2 of real blocks for launch shapes, then list capacities, then candidate bin edges (subsets of
-the box-side buckets present, at most `max_bins` bins), and keeps the fastest; results are stored per device name in `tuned.json` beside this file, which the library applies
-when it loads (`native.load`) and `device.batched_items` reads.
+the rest comes from the box each time; as many CTAs share an SM as hold the least list) trade resident reflections per
+SM against work per CTA. The tuner times pass 1 and pass 2 of real blocks for launch shapes, then list capacities, then
+candidate bin edges (subsets of the box-side buckets present, at most `max_bins` bins), and keeps a candidate that is
+faster than the kept one by more than MARGIN (several list capacities may give one launch the same plan). Results are
+stored per device name in `tuned.json` beside this file, which the library applies when it loads (`native.load`) and
+`device.batched_items` reads.
 
     python -m xpg_b200.tune [--workload config4|config2] [--max-bins 4]      (on the GPU)
 """
@@ -55,7 +57,8 @@ SHAPES = ({"wide_threads": 256, "pass1_stage_bytes": 48 * 1024}, {"wide_threads"
           {"wide_threads": 128, "pass1_stage_bytes": 96 * 1024})
 
 
-LIST_CAPS = (2048, 4096, 8192, 12288, 16384)
+LIST_CAPS = (512, 1024, 4096, 8192)
+MARGIN = 0.01
 CAP_DEFAULTS = {"pass2_list_cap": 2048, "pass2_list_cap_large": 2048}
 
 
@@ -68,7 +71,7 @@ def _apply(shape):
 def tune_round(picks, max_bins=4, reps=3, device="cuda", shapes=SHAPES, caps=LIST_CAPS):
     """Times the candidate launch shapes, then pass 2's fit-list capacities, then bin sets on one batched round of
     completed blocks. picks: list of (SweepRun, block) whose pass 1 and learning are done (their set entries valid).
-    Returns [(seconds, bins, shape)] fastest first."""
+    Returns [(seconds, bins, shape)], the kept one, then the others fastest first."""
     from . import native as N
     sets1, sets2, groups = [], [], []
     for k, (run, b) in enumerate(picks):
@@ -80,29 +83,31 @@ def tune_round(picks, max_bins=4, reps=3, device="cuda", shapes=SHAPES, caps=LIS
         groups.append((k, np.arange(rs.n), rs.bx, rs.Dz))
     t1, t2 = D.RowSetTable(sets1, device), D.RowSetTable(sets2, device)
     sides = np.concatenate([g[2] for g in groups])
-    out = []
+    out, kept = [], None
+
+    def trial(bins, shape):
+        """Times one candidate (its shape applied); it is kept when it is faster by more than the margin."""
+        nonlocal kept
+        launches = D.batched_items(groups, bins, device)
+        out.append((_time(lambda: (D.pass1_batched(t1, launches), D.pass2_batched(t2, launches)), reps), bins, shape))
+        if kept is None or out[-1][0] < (1.0 - MARGIN) * kept[0]:
+            kept = out[-1]
+
     base = candidates(sides, 1)[0]
     for shape in shapes:                 # launch shape first, on one bin of all sides
         _apply(shape)
-        launches = D.batched_items(groups, base, device)
-        out.append((_time(lambda: (D.pass1_batched(t1, launches), D.pass2_batched(t2, launches)), reps), base, shape))
-    best_shape = dict(min(out, key=lambda r: r[0])[2])
-    _apply(best_shape)
-    for key in ("pass2_list_cap", "pass2_list_cap_large"):   # pass 2's fit-list capacities (small, large boxes)
+        trial(base, shape)
+    for key in ("pass2_list_cap", "pass2_list_cap_large"):   # pass 2's least lists (small, large boxes)
+        best = dict(kept[2])
         for cap in caps:
-            shape = dict(best_shape, **{key: cap})
+            shape = dict(best, **{key: cap})
             _apply(shape)
-            launches = D.batched_items(groups, base, device)
-            out.append((_time(lambda: (D.pass1_batched(t1, launches), D.pass2_batched(t2, launches)), reps), base,
-                        shape))
-        best_shape = dict(min(out, key=lambda r: r[0])[2])
-        _apply(best_shape)
+            trial(base, shape)
+    best = dict(kept[2])
+    _apply(best)
     for bins in candidates(sides, max_bins)[1:]:
-        launches = D.batched_items(groups, bins, device)
-        t = _time(lambda: (D.pass1_batched(t1, launches), D.pass2_batched(t2, launches)), reps)
-        out.append((t, bins, best_shape))
-    out.sort(key=lambda r: r[0])
-    return out
+        trial(bins, best)
+    return [kept] + sorted((r for r in out if r is not kept), key=lambda r: r[0])
 
 
 def save(device_name, table, workload):
