@@ -441,8 +441,8 @@ constexpr int kGatherBatch = 4, kGatherFloatBatch = 8;
 // Dynamic shared memory of pass 1 for boxes up to max_bx pixels a side and max_dz bins with K neighbour columns: the
 // neighbours' frame masks (8P) | geometry scratch eps1, then the background template (4P) | eps2, then the img2 counts
 // (4P) | per pixel the number of clean foreground-frame voxels and the all-clean bit (P) | frame 64's neighbour bits,
-// the foreground pixels and the background ring's (a bit each) | foreground list | rocking-curve terms, then the clip candidates | the
-// neighbours' axis terms | staged shoebox.
+// the foreground pixels and the background ring's (a bit each) | foreground list | rocking-curve terms, then the clip
+// candidates | the neighbours' axis terms | staged shoebox.
 struct Pass1Layout {
     int Pm, cap, fgcap;
     size_t e1, e2, imgn, hi, fg, ring, fgl, scr, nbt, stage, bytes;
@@ -489,8 +489,8 @@ template <int NT> constexpr int min_ctas_pass1() { return 1024 / NT; }
 // row runs twice is one function. (Loads of the next batch ahead of the tests, in more registers, lost more by their
 // code than they hid: 13.9 ms in place of 12.1 for the sweep below at that stage.)
 //
-// Before and after: 107,446 rows of the 16M-pixel geometry (90 frames, 2.6e9 voxels) 14.2 -> 9.5 ms, 4,096 boxes of
-// 31 x 31 x 33 0.83 -> 0.48 ms, 40,001 of 9 x 9 x 5 0.90 -> 0.52 ms.
+// Before and after: 107,446 rows of the 16M-pixel geometry (90 frames, 2.6e9 voxels) 14.1 -> 9.3 ms, 4,096 boxes of
+// 31 x 31 x 33 0.82 -> 0.48 ms, 40,001 of 9 x 9 x 5 0.90 -> 0.52 ms.
 template <int NT, bool STAGED>
 __device__ __forceinline__ void pass1_row(const XiDetector& det_g, const XiRows& R, const XiBlock& B,
                                           const float* __restrict__ arena, const XiPass1Out& O, int row, int max_bx,
@@ -1080,7 +1080,7 @@ __global__ void __launch_bounds__(NT, min_ctas_pass1<NT>()) k_pass1_q(const XiRo
 // ==================================================================================================================
 // pass 2
 // ==================================================================================================================
-constexpr int kFitPix = 2048;       // pixels that may hold fitted voxels, listed per CTA, when not all of the box's can be
+constexpr int kFitPix = 2048;       // pixels that may hold fitted voxels, listed per CTA when not all of the box's can
 constexpr int kFitChunk = 9;        // frames of such a pixel that a thread takes
 constexpr int kFitWarp = 128;       // listed voxels that a warp of the fit takes
 
@@ -1166,15 +1166,16 @@ __device__ __forceinline__ void group_sum(double (&v)[NV], bool mid, bool end, i
 // Bound by instructions and by the latency of its serial steps, as pass 1. Only a few percent of a box's voxels enter
 // the fit, those where the profile exceeds a hundredth of its largest value, while every voxel's validity counts (for
 // the profile share on valid voxels). So the scan of the box tests validity alone (a compare a voxel, 17 loads in
-// flight: 10.3 ms for the sweep below, 10.8 with nine), and the pixels whose column can hold fitted voxels are listed and taken again, a thread a run of up to
-// nine frames. Six rounds of the fit then run on the compacted fitted voxels in few warps, with one barrier a round
-// (none for one warp) and only the sums the row needs; the other warps are done.
+// flight: 10.3 ms for the sweep below at that stage, 10.8 with nine), and the pixels whose column can hold fitted voxels
+// are listed and taken again, a thread a run of up to nine frames. Six rounds of the fit then run on the compacted fitted
+// voxels in few warps, with one barrier a round (none for one warp) and only the sums the row needs; the other warps are
+// done.
 // Where the list overflows, the runs that did not fit are taken from the box again in every round (the rows used to
 // scan their whole box).
 //
-// Before and after: 107,446 rows of the 16M-pixel geometry (90 frames, 500 fitted voxels a row) 17.0 -> 9.3 ms, 4,096
-// boxes of 31 x 31 x 33 (5,350 fitted) 2.89 -> 1.05 ms, 1,003 of 41 x 41 x 65 (21,000 fitted) 6.86 -> 1.36 ms, 40,001 of
-// 9 x 9 x 5 1.29 -> 0.89 ms.
+// Before and after: 107,446 rows of the 16M-pixel geometry (90 frames, 500 fitted voxels a row) 16.9 -> 8.8 ms, 4,096
+// boxes of 31 x 31 x 33 (5,350 fitted) 2.88 -> 1.02 ms, 1,003 of 41 x 41 x 65 (21,000 fitted) 6.86 -> 1.35 ms, 40,001 of
+// 9 x 9 x 5 1.28 -> 0.84 ms.
 template <int NT, bool STAGED>
 __device__ __forceinline__ void pass2_row(const XiDetector& det_g, const XiRows& R, const XiBlock& B,
                                           const float* __restrict__ arena, const float* __restrict__ prof,
@@ -2222,8 +2223,10 @@ int xi_gather(const XiFrames* F, const XiGatherRows* G, float* arena, int32_t* c
     const bool small = G->max_bx > 0 && G->max_bx <= (F->is_float ? kGatherSmallFloat : kGatherSmall);
     const int nt = small ? kGatherThreads / 2 : kGatherThreads;
     cudaStream_t s = (cudaStream_t)stream;
-    if (F->is_float && !small) k_gather<kGatherFloatBatch><<<nblk, nt, 0, s>>>(*F, *G, arena, cnt, G->order);
-    else k_gather<kGatherBatch><<<nblk, nt, 0, s>>>(*F, *G, arena, cnt, G->order);
+    if (F->is_float && !small)
+        k_gather<kGatherFloatBatch><<<nblk, nt, 0, s>>>(*F, *G, arena, cnt, G->order);
+    else
+        k_gather<kGatherBatch><<<nblk, nt, 0, s>>>(*F, *G, arena, cnt, G->order);
     return cuda_check("xi_gather");
 }
 
