@@ -284,9 +284,8 @@ class Workload:
 
 
 # DRAM bytes (read + write) per shoebox voxel of the pass kernels, from one ncu capture of a launch of the same
-# kernels on the config-2 geometry (a 20-frame block, `--workload config2-small`: the 2,597-reflection launch of
-# 31 x 31 x 33 boxes, 82.4 M voxels); the traffic of a launch here is that figure times its voxels
-DRAM_BYTES_PER_VOXEL = {"pass1": 5.060, "pass2": 4.432}
+# kernels (12,000 boxes of 23 x 23 x 33, 209.5 M voxels); the traffic of a launch here is that figure times its voxels
+DRAM_BYTES_PER_VOXEL = {"pass1": 4.578, "pass2": 4.407}
 
 
 def _parity(wl, res, n_min=500):
