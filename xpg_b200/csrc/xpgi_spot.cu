@@ -598,8 +598,10 @@ extern "C" size_t xi_spot_workspace(int n_frames, int ny, int nx) {
     if (n_frames < 0 || ny < 0 || nx < 0) return 0;
     const size_t n = (size_t)n_frames * ny * nx;
     const size_t flags = (n + 255) / 256 * 256;
-    // the first pass's flags (strong, or near a strong pixel; background), and its mean where a window may take tiles
-    return 2 * flags + (strip_ctas(true, n_frames, ny, nx, 12) < kWideCtas ? n * sizeof(float) : 0);
+    // the first pass's flags (strong, or near a strong pixel; background), and its mean for as many pixels as tiles are
+    // taken for (so that the scratch of a batch serves a shorter one)
+    const size_t most = (size_t)kWideCtas * (kCols - 4) * 12;
+    return 2 * flags + (n < most ? n : most) * sizeof(float);
 }
 
 extern "C" int xi_spot_strong(const float* img, int n_frames, int ny, int nx, float gain, const XiSpotParams* p,
