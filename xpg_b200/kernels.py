@@ -30,7 +30,7 @@ def _np(v):
     return np.asarray(v)
 
 
-# the tensors that have a numpy form; the others (bfloat16, float8, views with a pending conjugate or sign) are refused
+# the types of tensors that have a numpy form (bfloat16, float8 and views with a pending conjugate or sign have none)
 _TYPES = frozenset((torch.float64, torch.float32, torch.float16, torch.int64, torch.int32, torch.int16, torch.int8,
                     torch.uint64, torch.uint32, torch.uint16, torch.uint8, torch.bool, torch.complex64,
                     torch.complex128))
@@ -42,10 +42,9 @@ def _in(v):
     most of a call (4096 boxes of 31 x 31 x 33: 26.3 ms for the three passes, 3.8 ms of it kernels)."""
     if not (torch.is_tensor(v) and v.is_cuda):
         return _np(v)
-    if v.dtype not in _TYPES or v.is_neg() or v.is_conj():
-        raise TypeError(f"argument of type {v.dtype}" + (" with a pending sign or conjugate" if v.dtype in _TYPES else "")
-                        + " has no numpy form")
-    return v.detach()
+    if v.dtype not in _TYPES or v.is_neg() or (v.dtype.is_complex and v.is_conj()):
+        raise TypeError(f"a {v.dtype} tensor without a numpy form (its type, or a pending sign or conjugate)")
+    return v.detach() if v.requires_grad else v
 
 
 def _as(v, dtype):
